@@ -25,8 +25,8 @@ namespace bempp_b200 {
 
 void build_singular_pairs(GridT& g, SingularPairList& out);
 void build_tiles(const SpaceT& s, int tile, std::vector<int>& off, std::vector<int>& dofs,
-                 std::vector<uint8_t>& ldof, int& max_dofs, std::vector<uint8_t>& inc_off,
-                 std::vector<uint8_t>& inc_ent);
+                 std::vector<uint8_t>& ldof, int& max_dofs, int& max_half_dofs,
+                 std::vector<uint8_t>& inc_off, std::vector<uint8_t>& inc_ent);
 int scatter_tile_cells();
 cudaError_t launch_convert_to_single(const double* src, void* dst, size_t n_reals,
                                      cudaStream_t stream);
@@ -159,7 +159,8 @@ void ensure_space_device(SpaceT& s, int device) {
   std::vector<uint8_t> ldof;
   s.tile_cells = scatter_tile_cells();
   std::vector<uint8_t> inc_off, inc_ent;
-  build_tiles(s, s.tile_cells, off, tdofs, ldof, s.max_tile_dofs, inc_off, inc_ent);
+  build_tiles(s, s.tile_cells, off, tdofs, ldof, s.max_tile_dofs, s.max_chunk_dofs, inc_off,
+              inc_ent);
   s.d_tile_inc_off.upload(inc_off);
   s.d_tile_inc_ent.upload(inc_ent);
   s.ntiles = static_cast<int>(off.size()) - 1;
@@ -186,6 +187,7 @@ SpaceTiles space_tiles(const SpaceT& s) {
   t.tile_cells = s.tile_cells;
   t.ntiles = s.ntiles;
   t.max_tile_dofs = s.max_tile_dofs;
+  t.max_chunk_dofs = s.max_chunk_dofs;
   t.tile_dof_off = s.d_tile_off.as<int>();
   t.tile_dofs = s.d_tile_dofs.as<int>();
   t.cell_ldof = s.d_cell_ldof.as<uint8_t>();
@@ -450,15 +452,17 @@ void assemble_device(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& test, void* d
                              (test.grid->max_circumradius() + trial.grid->max_circumradius()) *
                              (1.0 + 1e-6);
   ra.small_phase = phase_bound <= 0.8 ? 1 : 0;
-  // one P1 / DP1 space, double layer or its adjoint, 6-point rule (Helmholtz: with the
-  // phases referenced to the pair): the pair (i, j) and the pair (j, i) share their
-  // kernel values, so both blocks of a tile pair come from one pass (one-launch assemblies
-  // only: a chunked host-memory assembly keeps the full tile grid, whose columns finish
-  // evenly through the chunks and go out by DMA meanwhile, where the tx >= sy half
+  // one P1 / DP1 space, double layer or its adjoint (mixed precision: the 6-point rule and,
+  // for Helmholtz, phases referenced to the pair): the pair (i, j) and the pair (j, i) share
+  // their kernel values, so both blocks of a tile pair come from one pass (one-launch
+  // assemblies only: a chunked host-memory assembly keeps the full tile grid, whose columns
+  // finish evenly through the chunks and go out by DMA meanwhile, where the tx >= sy half
   // finishes most columns only in its last chunks; measured on the 20,480-triangle
   // sphere, 16 chunks: 28.5 against 27.1 ms for the double layer)
-  if (&trial == &test && same_grid && (a.kernel == kLaplace || ra.small_phase) &&
-      (a.op == kDL || a.op == kADL) && test.nbasis == 3 && rule.npts == 6 && nchunks == 1)
+  const bool paired_kernel = ra.precision == kRegularFP64 ||
+                             (rule.npts == 6 && (a.kernel == kLaplace || ra.small_phase));
+  if (&trial == &test && same_grid && paired_kernel && (a.op == kDL || a.op == kADL) &&
+      test.nbasis == 3 && nchunks == 1)
     ra.symmetric = 2;
   a.tx_ge_sy = ra.symmetric != 0;
   if (ra.precision == kRegularMixed && nt > 0 && ns > 0) {
@@ -488,7 +492,7 @@ void assemble_device(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& test, void* d
     SingularPairList& pl = grid_pairs(*test.grid, device);
     const DeviceRules& dr = device_rules(device, order);
     rules = SingularRules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                          dr.w.as<double>()};
+                            dr.w.as<double>()};
     pairs = SingularPairs{static_cast<int>(pl.test_cell.size()), pl.d_test.as<int>(),
                           pl.d_trial.as<int>(), pl.d_config.as<int>()};
     pairs_ready = true;

@@ -116,11 +116,18 @@ __device__ __forceinline__ bool share_vertex(int a0, int a1, int a2, int b0, int
 // (1 - e)^(-1/2) = 1 + e/2 + 3e^2/8 + O(e^3) with e = 1 - a y^2, which cubes the
 // relative error of the seed.  Only used for distances between distinct quadrature
 // points (a > 0, far from the subnormal range).
+//
+// The correction multiplies the seed last, y (1 + e (1/2 + 3e/8)): no step reads three
+// different registers.  An FP64 FMA of three distinct register operands issues every 2.5
+// cycles on a B200's scheduler, one with a constant or a repeated operand every 2.03
+// (measured on chains of 64), so y + (y e)(1/2 + 3e/8), as many operations, cost more: a loop
+// of r^2, this root and a sum reached 73 % of the FP64 issue rate with four warps per
+// scheduler that way and 84 % this way.
 __device__ __forceinline__ double rsqrt_refined(double a) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
   const double e = fma(-a * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
+  return y * fma(e, fma(e, 0.375, 0.5), 1.0);
 }
 
 // sin(r) and cos(r) in FP64 for |r| <= pi/4: Taylor series up to r^17 and r^16
@@ -166,7 +173,7 @@ __device__ __forceinline__ void sincos_small(double t, double& s, double& c) {
   q = fma(q, z, -0.00019841269836043575);
   q = fma(q, z, 0.008333333333330467);
   q = fma(q, z, -0.16666666666666663);
-  s = fma(t * z, q, t);
+  s = t * fma(z, q, 1.0);
 }
 
 // sin(t) and cos(t) in FP64 for moderate |t| (the phases k r of boundary-element
@@ -185,6 +192,80 @@ __device__ __forceinline__ void sincos_cw(double t, double& s, double& c) {
   s = (q == 0) ? sr : (q == 1) ? cr : (q == 2) ? -sr : -cr;
 }
 
+// sincos_small of N arguments, step by step.
+template <int N>
+__device__ __forceinline__ void sincos_small_n(const double t[N], double s[N], double c[N]) {
+  constexpr double P[6] = {2.0657616391477202e-09,  -2.755574396426964e-07, 2.4801582078024058e-05,
+                           -0.0013888888881056654, 0.04166666666662371,    -0.4999999999999996};
+  constexpr double Q[6] = {1.5912864224903485e-10, -2.5051057394492127e-08, 2.7557315738586845e-06,
+                           -0.00019841269836043575, 0.008333333333330467,   -0.16666666666666663};
+  double z[N], p[N], q[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) z[i] = t[i] * t[i];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    p[i] = P[0];
+    q[i] = Q[0];
+  }
+#pragma unroll
+  for (int j = 1; j < 6; ++j) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[i] = fma(p[i], z[i], P[j]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) q[i] = fma(q[i], z[i], Q[j]);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) c[i] = fma(z[i], p[i], 1.0);
+#pragma unroll
+  for (int i = 0; i < N; ++i) s[i] = t[i] * fma(z[i], q[i], 1.0);
+}
+
+// sin(t), cos(t) of N arguments of any size: reduction by pi/2 (the multiple read from the
+// low word of t (2/pi) + 1.5 2^52, two-part pi/2, each step one FMA), sincos_small_n, the
+// quadrant's exchange by integer operations.  18 FP64 operations; absolute error about
+// 2.5e-16.  Arguments beyond 2^43 (whose last digit is worth more than 1e-3) are brought
+// down by multiples of 2 pi first, so that the result is a point of the unit circle for
+// every t.
+template <int N>
+__device__ __forceinline__ void sincos_any_n(const double t[N], double s[N], double c[N]) {
+  double r[N], n[N];
+  int q[N];
+  bool huge = false;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    r[i] = t[i];
+    huge |= static_cast<unsigned>(__double2hiint(t[i]) & 0x7fffffff) >= 0x42a00000u;
+  }
+  if (huge) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      while (fabs(r[i]) >= 8796093022208.0 && fabs(r[i]) <= 1.7e308)
+        r[i] = fma(-rint(r[i] * 0.15915494309189533577), 6.2831853071795864769, r[i]);
+  }
+  const double big = 6755399441055744.0;  // 1.5 * 2^52
+#pragma unroll
+  for (int i = 0; i < N; ++i) n[i] = fma(r[i], 0.63661977236758134308, big);
+#pragma unroll
+  for (int i = 0; i < N; ++i) q[i] = __double2loint(n[i]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) n[i] -= big;
+#pragma unroll
+  for (int i = 0; i < N; ++i) r[i] = fma(-n[i], 1.5707963267948966192, r[i]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) r[i] = fma(-n[i], 6.1232339957367660359e-17, r[i]);
+  double sr[N], cr[N];
+  sincos_small_n<N>(r, sr, cr);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double a = (q[i] & 1) ? cr[i] : sr[i], b = (q[i] & 1) ? sr[i] : cr[i];
+    s[i] = __hiloint2double(__double2hiint(a) ^ ((q[i] & 2) << 30), __double2loint(a));
+    c[i] = __hiloint2double(__double2hiint(b) ^ (((q[i] + 1) & 2) << 30), __double2loint(b));
+  }
+}
+__device__ __forceinline__ void sincos_any(double t, double& s, double& c) {
+  sincos_any_n<1>(&t, &s, &c);
+}
+
 // a^(-3/2) for normal positive FP64 a: the rsqrt.approx.ftz.f64 seed y refined by the
 // series (1 - e)^(-3/2) = 1 + 3e/2 + 15e^2/8 + O(e^3) with e = 1 - a y^2 (the inverse cube
 // of a distance from its square, for double-layer kernels).
@@ -193,8 +274,7 @@ __device__ __forceinline__ double rinv3_refined(double a) {
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
   const double y2 = y * y;
   const double e = fma(-a, y2, 1.0);
-  const double y3 = y2 * y;
-  return fma(y3 * e, fma(e, 1.875, 1.5), y3);
+  return (y2 * y) * fma(e, fma(e, 1.875, 1.5), 1.0);
 }
 
 // Lagrange basis of NB functions (1: degree 0, 3: degree 1, 6: degree 2 in ndelement's

@@ -81,6 +81,7 @@ struct SpaceTiles {
   int tile_cells;           // cells per tile
   int ntiles;
   int max_tile_dofs;
+  int max_chunk_dofs;       // most DOFs of 16 consecutive cells (half a tile)
   const int* tile_dof_off;  // ntiles + 1
   const int* tile_dofs;     // global DOF numbers of each tile, ascending
   const uint8_t* cell_ldof; // ncells * nbasis local (in-tile) DOF indices
@@ -97,6 +98,12 @@ cudaError_t launch_regular_scatter(const CellSet& test, const SpaceTiles& ttiles
                                    const CellSet& trial, const SpaceTiles& stiles,
                                    const RegularRule& rule, const RegularArgs& a,
                                    cudaStream_t stream);
+
+// The FP64 kernels of DP0 / P1 / DP1 spaces (regular_fp64.cu and the files of the same
+// prefix): stores (direct, DP0 x DP0) or adds into the zeroed output.
+cudaError_t launch_regular_fp64(const CellSet& test, const SpaceTiles& tt, const CellSet& trial,
+                                const SpaceTiles& st, const RegularRule& rule,
+                                const RegularArgs& a, cudaStream_t stream, bool direct);
 
 // Singular (Duffy) rules of all 28 adjacency configurations, concatenated.
 struct SingularRules {

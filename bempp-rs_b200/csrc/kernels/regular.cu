@@ -1,4 +1,6 @@
-// Regular (non-singular) quadrature of all operators and space pairs, FP64 or mixed.
+// Regular (non-singular) quadrature of all operators and space pairs in mixed precision, the
+// FP64 near pairs of mixed assemblies, and the FP64 degree-2 tiles (FP64 on spaces of degree
+// 0 and 1: regular_fp64.cuh).
 //
 // Replaces the hot loop of bempp-rs assemble_nonsingular_part / assemble_batch_nonadjacent
 // (src/boundary_assemblers.rs:396-521,689-773) and NonsingularCellPairAssemblerWithTest-
@@ -126,7 +128,7 @@ __device__ __forceinline__ void finish_block(const Tile& T, int it, const Tile& 
 enum F64Phase : int { kF64Sincos = 0, kF64Reduced = 1, kF64Referenced = 2 };
 
 // FP64 local block, test points outermost (every operator but the Laplace adjoint double
-// layer).
+// layer): near pairs and degree-2 spaces.
 template <int QT, int KER, int OP, int NBT, int NBS, bool kUnroll, int FPH>
 __device__ __forceinline__ void block_fp64_pq(const Tile& T, int it, const Tile& S, int js,
                                         const RegularRule& rule, double k,
@@ -325,155 +327,6 @@ __device__ __forceinline__ void block_fp64(const Tile& T, int it, const Tile& S,
     block_fp64_adl_laplace<QT, NBT, NBS, kUnroll>(T, it, S, js, rule, ore, oim);
   else
     block_fp64_pq<QT, KER, OP, NBT, NBS, kUnroll, FPH>(T, it, S, js, rule, k, ore, oim);
-}
-
-// Laplace double layer of a cell pair in both orders, FP64, for one P1 / DP1 space on both
-// sides (the same rule on both cells): from one 1/r^3 per point pair (x_p in cell i of the
-// test tile, y_q in cell j of the trial tile)
-//   dij[a][b] = DL(test i, trial j)_ab = sum_p w_p phi_a(p) (x_p - y).n_j sum_q w_q phi_b(q) / r^3
-//   dji[a][b] = DL(test j, trial i)_ba = sum_p w_p phi_a(p) sum_q w_q phi_b(q) (y_q - x).n_i / r^3
-// ((x - y).n is constant over the plane of the normal's cell, in the tangent coordinates of
-// block_fp64_pq).  Both trial-point sums close per test point; the reverse order's normal
-// factor is formed per point pair (3 FP64 operations), which keeps 15 fewer doubles live
-// than summing per trial point and applying it at the end (8 % faster at 20,480 cells).
-// The adjoint double layer is the same pair of blocks swapped: ADL(i, j)_ab = DL(j, i)_ba.
-template <int Q>
-__device__ __forceinline__ void block_fp64_dl_pair(const Tile& T, int it, const Tile& S,
-                                                        int js, const RegularRule& rule,
-                                                        double dij[3][3], double dji[3][3]) {
-  static_assert(Q > 0, "the paired double layer needs a compile-time rule size");
-  const double dcx = T.G(fCx, it) - S.G(fCx, js), dcy = T.G(fCy, it) - S.G(fCy, js),
-               dcz = T.G(fCz, it) - S.G(fCz, js);
-  const double njx = S.G(fNx, js), njy = S.G(fNy, js), njz = S.G(fNz, js);
-  const double nix = T.G(fNx, it), niy = T.G(fNy, it), niz = T.G(fNz, it);
-  const double f0 = dcx * njx + dcy * njy + dcz * njz;
-  const double f1 = T.G(fT0x, it) * njx + T.G(fT0y, it) * njy + T.G(fT0z, it) * njz;
-  const double f2 = T.G(fT1x, it) * njx + T.G(fT1y, it) * njy + T.G(fT1z, it) * njz;
-  const double g0 = -(dcx * nix + dcy * niy + dcz * niz);
-  const double g1 = S.G(fT0x, js) * nix + S.G(fT0y, js) * niy + S.G(fT0z, js) * niz;
-  const double g2 = S.G(fT1x, js) * nix + S.G(fT1y, js) * niy + S.G(fT1z, js) * niz;
-  double bij[3][3], bji[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) bij[a][b] = bji[a][b] = 0.0;
-#pragma unroll 1
-  for (int p = 0; p < Q; ++p) {
-    const double x0 = T.P(p, 0, it), x1 = T.P(p, 1, it), x2 = T.P(p, 2, it);
-    double u0 = 0.0, u1 = 0.0, u2 = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const double dx = x0 - S.P(q, 0, js), dy = x1 - S.P(q, 1, js), dz = x2 - S.P(q, 2, js);
-      const double kern = rinv3_refined(dx * dx + dy * dy + dz * dz);
-      u0 = fma(kern, rule.wphi[0][q], u0);
-      u1 = fma(kern, rule.wphi[1][q], u1);
-      u2 = fma(kern, rule.wphi[2][q], u2);
-      const double kb = kern * fma(rule.u[q], g1, fma(rule.v[q], g2, g0));
-      v0 = fma(kb, rule.wphi[0][q], v0);
-      v1 = fma(kb, rule.wphi[1][q], v1);
-      v2 = fma(kb, rule.wphi[2][q], v2);
-    }
-    const double ap = fma(rule.u[p], f1, fma(rule.v[p], f2, f0));
-    const double c[3] = {rule.wphi[0][p], rule.wphi[1][p], rule.wphi[2][p]};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double e = c[a] * ap;
-      bij[a][0] = fma(e, u0, bij[a][0]);
-      bij[a][1] = fma(e, u1, bij[a][1]);
-      bij[a][2] = fma(e, u2, bij[a][2]);
-      bji[a][0] = fma(c[a], v0, bji[a][0]);
-      bji[a][1] = fma(c[a], v1, bji[a][1]);
-      bji[a][2] = fma(c[a], v2, bji[a][2]);
-    }
-  }
-  const double sc = T.G(fJdet, it) * S.G(fJdet, js) * kInv4Pi;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      dij[a][b] = bij[a][b] * sc;
-      dji[a][b] = bji[a][b] * sc;
-    }
-}
-
-// The Helmholtz double layer of a cell pair in both orders, FP64, as block_fp64_dl_pair:
-// one kernel value e^{ikr} (1 - ikr) / r^3 per point pair, the phase referenced to the
-// pair (e^{ikr} = e^{ik r0} e^{ik (r - r0)}, |k (r - r0)| <= 0.8 checked on the host), both
-// blocks rotated by e^{ik r0} at the end.
-template <int Q>
-__device__ __forceinline__ void block_fp64_dl_pair_helmholtz(
-    const Tile& T, int it, const Tile& S, int js, const RegularRule& rule, double k,
-    double dij_re[3][3], double dij_im[3][3], double dji_re[3][3], double dji_im[3][3]) {
-  static_assert(Q > 0, "the paired double layer needs a compile-time rule size");
-  const double dcx = T.G(fCx, it) - S.G(fCx, js), dcy = T.G(fCy, it) - S.G(fCy, js),
-               dcz = T.G(fCz, it) - S.G(fCz, js);
-  const double njx = S.G(fNx, js), njy = S.G(fNy, js), njz = S.G(fNz, js);
-  const double nix = T.G(fNx, it), niy = T.G(fNy, it), niz = T.G(fNz, it);
-  const double f0 = dcx * njx + dcy * njy + dcz * njz;
-  const double f1 = T.G(fT0x, it) * njx + T.G(fT0y, it) * njy + T.G(fT0z, it) * njz;
-  const double f2 = T.G(fT1x, it) * njx + T.G(fT1y, it) * njy + T.G(fT1z, it) * njz;
-  const double g0 = -(dcx * nix + dcy * niy + dcz * niz);
-  const double g1 = S.G(fT0x, js) * nix + S.G(fT0y, js) * niy + S.G(fT0z, js) * niz;
-  const double g2 = S.G(fT1x, js) * nix + S.G(fT1y, js) * niy + S.G(fT1z, js) * niz;
-  const double r0sq = dcx * dcx + dcy * dcy + dcz * dcz;
-  const double kr0 = k * (r0sq * rsqrt_refined(r0sq));
-  double bij_re[3][3], bij_im[3][3], bji_re[3][3], bji_im[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) bij_re[a][b] = bij_im[a][b] = bji_re[a][b] = bji_im[a][b] = 0.0;
-#pragma unroll 1
-  for (int p = 0; p < Q; ++p) {
-    const double x0 = T.P(p, 0, it), x1 = T.P(p, 1, it), x2 = T.P(p, 2, it);
-    double ur[3] = {0.0, 0.0, 0.0}, ui[3] = {0.0, 0.0, 0.0};
-    double vr[3] = {0.0, 0.0, 0.0}, vi[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const double dx = x0 - S.P(q, 0, js), dy = x1 - S.P(q, 1, js), dz = x2 - S.P(q, 2, js);
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      const double rinv = rsqrt_refined(r2);
-      const double r = r2 * rinv, kr = k * r;
-      double sn, cs;
-      sincos_small(fma(k, r, -kr0), sn, cs);  // e^{ik (r - r0)}
-      const double f = rinv * rinv * rinv;
-      const double kre = f * fma(kr, sn, cs), kim = f * fma(-kr, cs, sn);
-      const double bq = fma(rule.u[q], g1, fma(rule.v[q], g2, g0));
-      const double bre = kre * bq, bim = kim * bq;
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const double w = rule.wphi[b][q];
-        ur[b] = fma(kre, w, ur[b]);
-        ui[b] = fma(kim, w, ui[b]);
-        vr[b] = fma(bre, w, vr[b]);
-        vi[b] = fma(bim, w, vi[b]);
-      }
-    }
-    const double ap = fma(rule.u[p], f1, fma(rule.v[p], f2, f0));
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double c = rule.wphi[a][p], e = c * ap;
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        bij_re[a][b] = fma(e, ur[b], bij_re[a][b]);
-        bij_im[a][b] = fma(e, ui[b], bij_im[a][b]);
-        bji_re[a][b] = fma(c, vr[b], bji_re[a][b]);
-        bji_im[a][b] = fma(c, vi[b], bji_im[a][b]);
-      }
-    }
-  }
-  double ps, pc;
-  sincos_cw(kr0, ps, pc);
-  const double sc = T.G(fJdet, it) * S.G(fJdet, js) * kInv4Pi;
-  const double cr = pc * sc, ci = ps * sc;  // e^{ik r0} jdet_i jdet_j / (4 pi)
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      dij_re[a][b] = bij_re[a][b] * cr - bij_im[a][b] * ci;
-      dij_im[a][b] = bij_re[a][b] * ci + bij_im[a][b] * cr;
-      dji_re[a][b] = bji_re[a][b] * cr - bji_im[a][b] * ci;
-      dji_im[a][b] = bji_re[a][b] * ci + bji_im[a][b] * cr;
-    }
 }
 
 // Per-pair constants of the FP32 far-pair quadrature.
@@ -993,35 +846,29 @@ __device__ __forceinline__ void mirror_put(double* mir, int it, int js, double r
 // skipped (FP32 far pairs only; near_pairs_fp64 integrates the near ones).
 enum NearMode : int { kNearInKernel = 0, kNearMasked = 1 };
 
-// Resident CTAs per SM the register allocation must allow: 5 for the FP64 Laplace
-// hypersingular kernel (it fits in 96 registers without spills), 6 for the mixed
-// Helmholtz DP0 kernels (80 registers; with no FP64 points in their tiles six CTAs also
-// fit in shared memory), 3 for the paired FP64 Helmholtz double layer (168 registers; at
-// 128 it spills 228 bytes, and four CTAs per SM ran 17 % slower), 4 elsewhere (the paired
-// Laplace double layer too: at 128 registers it spills 48 bytes; the paired mixed
-// Helmholtz one, which stages the real and imaginary parts of its blocks in turn to fit
-// four CTAs in shared memory, needs 127 registers without spills).
-template <int KER, int OP, bool MIXED, bool DIRECT, bool PAIRED = false>
+// Resident CTAs per SM the register allocation must allow: 6 for the mixed Helmholtz DP0
+// kernels (80 registers; with no FP64 points in their tiles six CTAs also fit in shared
+// memory), 4 elsewhere (the paired mixed Helmholtz double layer, which stages the real and
+// imaginary parts of its blocks in turn to fit four CTAs in shared memory, needs 127
+// registers without spills).
+template <int KER, bool MIXED, bool DIRECT>
 constexpr int min_ctas() {
-  return (PAIRED && KER == kHelmholtz && !MIXED)   ? 3
-         : (KER == kLaplace && OP == kHS && !MIXED) ? 5
-         : (MIXED && DIRECT && KER == kHelmholtz)   ? 6
-                                                    : 4;
+  return MIXED && DIRECT && KER == kHelmholtz ? 6 : 4;
 }
 
-// PAIRED (Laplace DL / ADL, FP64, one P1 / DP1 space on both sides, Q = 6): the tile
-// pairs tx >= sy, each off-diagonal one integrated in both orders from one evaluation of
-// the kernel per point pair (block_fp64_dl_pair), the (sy, tx) blocks accumulated
-// separately and added at the transposed entries.
+// PAIRED (DL / ADL, mixed, one P1 / DP1 space on both sides, Q = 6): the tile pairs tx >=
+// sy, each off-diagonal one integrated in both orders from one evaluation of the kernel
+// per point pair (block_fp32_dl_pair), the (sy, tx) blocks accumulated separately and added
+// at the transposed entries.
 template <int QT, int KER, int OP, int NBT, int NBS, bool MIXED, bool DIRECT, int PH, int NM,
           bool PAIRED = false>
-__global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAIRED>())
+__global__ void __launch_bounds__(kThreads, min_ctas<KER, MIXED, DIRECT>())
     regular_tiles(CellSet test, SpaceTiles tt, CellSet trial, SpaceTiles st, RegularRule rule,
                   double k, int same_grid, double* __restrict__ out, int64_t ld, int tile_y0,
-                  int tile_y1, NearArgs near, int symmetric, int acc_copies) {
+                  int tile_y1, NearArgs near, int symmetric) {
   static_assert(!PAIRED || ((OP == kDL || OP == kADL) && NBT == 3 && NBS == 3 && !DIRECT &&
                             QT == 6 && (KER == kLaplace || PH == kPhaseSmall) &&
-                            (!MIXED || NM == kNearMasked)),
+                            MIXED && NM == kNearMasked),
                 "paired blocks: DL / ADL, P1 / DP1, 6-point rule (Helmholtz: phases "
                 "referenced to the pair; mixed: near pairs masked)");
   constexpr bool kC = KER == kHelmholtz;
@@ -1035,13 +882,6 @@ __global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAI
   // complex blocks gathered through one real stage, real parts first (paired mixed
   // Helmholtz: four CTAs per SM fit in shared memory)
   constexpr bool kSplitStage = kGather && kC && PAIRED && MIXED;
-  // real FP64 P1 blocks (not the hypersingular kernel, which keeps 5 CTAs per SM; not the
-  // mixed kernels, whose larger tiles would then limit the CTAs per SM): one accumulator
-  // per warp, updated with plain adds, summed at the flush
-  constexpr int kAccMax = (kGather && !kC && !MIXED && OP != kHS && !PAIRED) ? kWarps : 1;
-  // the host passes 1 when kAccMax copies of the largest DOF block do not fit in shared
-  // memory (DP1 x DP1: 96 x 96 DOFs per tile pair); the warps then add with atomics
-  const int kAcc = kAccMax > 1 && acc_copies > 1 ? kAccMax : 1;
   const int Q = QT > 0 ? QT : rule.npts;
   // symmetric operator on one space (single layer, hypersingular): only the tile pairs with
   // tx >= sy are computed, the blocks with tx > sy also written transposed
@@ -1073,7 +913,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAI
     cap = tt.max_tile_dofs * st.max_tile_dofs;
     acc_re = reinterpret_cast<double*>(cursor);
     acc_im = acc_re + cap;
-    cursor += sizeof(double) * cap * (kC ? 2 : 1) * kAcc;
+    cursor += sizeof(double) * cap * (kC ? 2 : 1);
   }
   // PAIRED: the (sy, tx) blocks, indexed as acc_re (test-tile DOF + ndt * trial-tile DOF),
   // imaginary parts (Helmholtz) cap further on
@@ -1112,11 +952,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAI
     stage_tile_bulk(S, trial, sj0, Q, kRel, mbar, kPts);
   }
   if (!DIRECT) {
-    for (int w = 0; w < kAcc; ++w)
-      for (int idx = threadIdx.x; idx < ndt * nds; idx += kThreads) {
-        acc_re[w * cap + idx] = 0.0;
-        if (kC) acc_im[idx] = 0.0;
-      }
+    for (int idx = threadIdx.x; idx < ndt * nds; idx += kThreads) {
+      acc_re[idx] = 0.0;
+      if (kC) acc_im[idx] = 0.0;
+    }
     if (PAIRED)
       for (int idx = threadIdx.x; idx < ndt * nds; idx += kThreads) {
         acc_t[idx] = 0.0;
@@ -1182,24 +1021,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAI
             block_fp32_dl_pair<QT, KER>(T, it, S, js, rule, k, ore, oim, otr, oti);
           else
             block_fp32_dl_pair<QT, KER>(T, it, S, js, rule, k, otr, oti, ore, oim);
-        } else if constexpr (PAIRED) {
-          // DL: (i, j) block here, (j, i) at the transposed entries; ADL: swapped
-          if constexpr (KER == kLaplace) {
-#pragma unroll
-            for (int a = 0; a < NBT; ++a)
-#pragma unroll
-              for (int b = 0; b < NBS; ++b) oim[a][b] = oti[a][b] = 0.0;  // real blocks
-            if (OP == kDL)
-              block_fp64_dl_pair<QT>(T, it, S, js, rule, ore, otr);
-            else
-              block_fp64_dl_pair<QT>(T, it, S, js, rule, otr, ore);
-          } else {
-            if (OP == kDL)
-              block_fp64_dl_pair_helmholtz<QT>(T, it, S, js, rule, k, ore, oim, otr, oti);
-            else
-              block_fp64_dl_pair_helmholtz<QT>(T, it, S, js, rule, k, otr, oti, ore, oim);
-          }
-        } else if (MIXED) {
+        } else if constexpr (MIXED) {
           block_fp32<QT, KER, OP, NBT, NBS, PH>(T, it, S, js, rule, k, ore, oim);
         } else {
           block_fp64<QT, KER, OP, NBT, NBS, true,
@@ -1253,12 +1075,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAI
 #pragma unroll
         for (int b = 0; b < NBS; ++b) {
           const int idx = d + ndt * S.ldof[b * kTile + js];
-          if (kAcc > 1) {
-            acc[warp * cap + idx] += g_re[b];  // this warp's copy; distinct per lane
-          } else {
-            atomicAdd(acc + idx, g_re[b]);
-            if (kC && !kSplitStage) atomicAdd(acci + idx, g_im[b]);
-          }
+          atomicAdd(acc + idx, g_re[b]);
+          if (kC && !kSplitStage) atomicAdd(acci + idx, g_im[b]);
         }
       }
       __syncwarp();
@@ -1307,9 +1125,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<KER, OP, MIXED, DIRECT, PAI
     for (int idx = threadIdx.x; idx < ndt * nds; idx += kThreads) {
       const int a = idx % ndt, b = idx / ndt;
       const int64_t o = static_cast<int64_t>(sdofs[b]) * ld + tdofs[a];
-      double re = acc_re[idx];
-#pragma unroll
-      for (int w = 1; w < kAcc; ++w) re += acc_re[w * cap + idx];
+      const double re = acc_re[idx];
       // symmetric, tx > sy: the same value at the transposed entry
       const int64_t om = static_cast<int64_t>(tdofs[a]) * ld + sdofs[b];
       if (kC && PAIRED) {
@@ -1679,31 +1495,11 @@ template <int QT, int KER, int OP, int NBT, int NBS, bool MIXED, bool DIRECT, in
 cudaError_t launch_mode(const CellSet& test, const SpaceTiles& tt, const CellSet& trial,
                         const SpaceTiles& st, const RegularRule& rule, const RegularArgs& a,
                         int ty0, int ty1, cudaStream_t stream) {
-  // accumulator copies: one per warp for the real FP64 P1 blocks; PAIRED: one for the
-  // (tx, sy) and one for the (sy, tx) blocks
-  constexpr int kAcc = PAIRED ? 2
-                              : (!DIRECT && NBT == 3 && KER != kHelmholtz && !MIXED && OP != kHS)
-                                    ? kWarps
-                                    : 1;
-  auto bytes = [&](int copies) {
-    return smem_bytes(rule.npts, MIXED, MIXED && NM == kNearInKernel, DIRECT, KER == kHelmholtz,
-                      tt.max_tile_dofs, st.max_tile_dofs, NBT, NBS, copies, a.symmetric != 0,
-                      !MIXED || NM == kNearInKernel,
-                      !DIRECT && NBT == 3 && KER == kHelmholtz && PAIRED && MIXED);
-  };
-  int copies = kAcc;
-  size_t smem = bytes(copies);
-  if (copies == kWarps) {
-    int device = 0, limit = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess)
-      e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    if (e != cudaSuccess) return e;
-    if (smem > static_cast<size_t>(limit)) {  // one shared accumulator, atomic adds
-      copies = 1;
-      smem = bytes(1);
-    }
-  }
+  // accumulators: PAIRED has one for the (tx, sy) and one for the (sy, tx) blocks
+  const size_t smem = smem_bytes(rule.npts, MIXED, MIXED && NM == kNearInKernel, DIRECT, KER == kHelmholtz,
+                                 tt.max_tile_dofs, st.max_tile_dofs, NBT, NBS, PAIRED ? 2 : 1,
+                                 a.symmetric != 0, !MIXED || NM == kNearInKernel,
+                                 !DIRECT && NBT == 3 && KER == kHelmholtz && PAIRED && MIXED);
   auto fn = regular_tiles<QT, KER, OP, NBT, NBS, MIXED, DIRECT, PH, NM, PAIRED>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
@@ -1721,7 +1517,7 @@ cudaError_t launch_mode(const CellSet& test, const SpaceTiles& tt, const CellSet
   }
   fn<<<grid, kThreads, smem, stream>>>(test, tt, trial, st, rule, a.k, a.same_grid,
                                        static_cast<double*>(a.out), a.ld, ty0, ty1, a.near,
-                                       a.symmetric, copies);
+                                       a.symmetric);
   return cudaGetLastError();
 }
 
@@ -1764,23 +1560,7 @@ cudaError_t launch_one(const CellSet& test, const SpaceTiles& tt, const CellSet&
   if (ny <= 0) return cudaSuccess;
   const int ty0 = a.trial_tile0, ty1 = a.trial_tile0 + ny;
   if constexpr (!MIXED) {
-    if (a.symmetric == 2) {
-      // one P1 / DP1 space, DL / ADL: both orders of each pair from one kernel evaluation
-      // (the host asks for it only there, for Helmholtz only with phases referenced to the
-      // pair)
-      if constexpr ((OP == kDL || OP == kADL) && NBT == 3 && NBS == 3 && !DIRECT && QT == 6) {
-        if (KER == kHelmholtz && !a.small_phase) return cudaErrorInvalidValue;
-        return launch_mode<QT, KER, OP, NBT, NBS, false, DIRECT, kPhaseSmall, kNearInKernel, true>(
-            test, tt, trial, st, rule, a, ty0, ty1, stream);
-      } else {
-        return cudaErrorInvalidValue;
-      }
-    }
-    // FP64 Helmholtz: phases referenced to the pair (kPhaseSmall) when the host's bound
-    // allows it, else CUDA's sincos of every phase
-    if (KER == kHelmholtz && !a.small_phase)
-      return launch_mode<QT, KER, OP, NBT, NBS, false, DIRECT, kPhaseGeneral, kNearInKernel>(
-          test, tt, trial, st, rule, a, ty0, ty1, stream);
+    if (a.symmetric == 2) return cudaErrorInvalidValue;
     return launch_mode<QT, KER, OP, NBT, NBS, false, DIRECT, kPhaseSmall, kNearInKernel>(
         test, tt, trial, st, rule, a, ty0, ty1, stream);
   } else {
@@ -1829,21 +1609,22 @@ template <int QT, int KER, int OP, bool MIXED>
 cudaError_t launch_spaces(const CellSet& test, const SpaceTiles& tt, const CellSet& trial,
                           const SpaceTiles& st, const RegularRule& rule, const RegularArgs& a,
                           cudaStream_t stream, bool direct) {
-  if (direct) {
-    if (OP == kHS) return cudaErrorInvalidValue;
-    return launch_one<QT, KER, OP == kHS ? kSL : OP, 1, 1, MIXED, true>(test, tt, trial, st, rule, a, stream);
-  }
-  if (tt.nbasis == 1 && st.nbasis == 1)
-    return launch_one<QT, KER, OP, 1, 1, MIXED, false>(test, tt, trial, st, rule, a, stream);
-  if (tt.nbasis == 1 && st.nbasis == 3)
-    return launch_one<QT, KER, OP, 1, 3, MIXED, false>(test, tt, trial, st, rule, a, stream);
-  if (tt.nbasis == 3 && st.nbasis == 1)
-    return launch_one<QT, KER, OP, 3, 1, MIXED, false>(test, tt, trial, st, rule, a, stream);
-  if (tt.nbasis == 3 && st.nbasis == 3)
-    return launch_one<QT, KER, OP, 3, 3, MIXED, false>(test, tt, trial, st, rule, a, stream);
-  if constexpr (!MIXED && KER == kLaplace && OP != kHS) {
+  if constexpr (MIXED) {
+    if (direct) {
+      if (OP == kHS) return cudaErrorInvalidValue;
+      return launch_one<QT, KER, OP == kHS ? kSL : OP, 1, 1, true, true>(test, tt, trial, st, rule, a, stream);
+    }
+    if (tt.nbasis == 1 && st.nbasis == 1)
+      return launch_one<QT, KER, OP, 1, 1, true, false>(test, tt, trial, st, rule, a, stream);
+    if (tt.nbasis == 1 && st.nbasis == 3)
+      return launch_one<QT, KER, OP, 1, 3, true, false>(test, tt, trial, st, rule, a, stream);
+    if (tt.nbasis == 3 && st.nbasis == 1)
+      return launch_one<QT, KER, OP, 3, 1, true, false>(test, tt, trial, st, rule, a, stream);
+    if (tt.nbasis == 3 && st.nbasis == 3)
+      return launch_one<QT, KER, OP, 3, 3, true, false>(test, tt, trial, st, rule, a, stream);
+  } else if constexpr (KER == kLaplace && OP != kHS) {
     // degree 2 on both sides (P2 / DP2), FP64
-    if (tt.nbasis == 6 && st.nbasis == 6)
+    if (!direct && tt.nbasis == 6 && st.nbasis == 6)
       return launch_one<QT, KER, OP, 6, 6, false, false>(test, tt, trial, st, rule, a, stream);
   }
   return cudaErrorInvalidValue;
@@ -1876,6 +1657,8 @@ cudaError_t dispatch(const CellSet& test, const SpaceTiles& tt, const CellSet& t
                      cudaStream_t stream, bool direct) {
   if (test.ncells <= 0 || trial.ncells <= 0) return cudaSuccess;
   const bool mixed = a.precision == kRegularMixed;
+  if (!mixed && tt.nbasis <= 3 && st.nbasis <= 3)
+    return launch_regular_fp64(test, tt, trial, st, rule, a, stream, direct);
   if (rule.npts == 6)
     return mixed ? launch_kernel<6, true>(test, tt, trial, st, rule, a, stream, direct)
                  : launch_kernel<6, false>(test, tt, trial, st, rule, a, stream, direct);

@@ -1,0 +1,12 @@
+// Regular quadrature, FP64, Laplace, the 6-point rule (see regular_fp64.cuh).
+#include "regular_fp64.cuh"
+
+namespace bempp_b200 {
+
+cudaError_t launch_fp64_laplace6(const CellSet& test, const SpaceTiles& tt, const CellSet& trial,
+                                 const SpaceTiles& st, const RegularRule& rule,
+                                 const RegularArgs& a, cudaStream_t stream, bool direct) {
+  return fp64::launch_op<true, kLaplace, fp64::kReferenced>(test, tt, trial, st, rule, a, stream, direct);
+}
+
+}  // namespace bempp_b200
