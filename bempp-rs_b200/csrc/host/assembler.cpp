@@ -56,7 +56,25 @@ int current_device() {
 // Duffy rules per (device, order), shared by all assemblers.
 struct DeviceRules {
   DeviceBuffer offset, test_xi, trial_xi, w;
-  int total = 0;
+  int total = 0, order = 0;
+  // triangles: directions and radii
+  DeviceBuffer dir_offset, coef, rho, weights[2][4], share, raw, roles, cell_series[2];
+  SeriesRules series[2];
+  SingularRules view() const {
+    SingularRules r{offset.as<int>(), test_xi.as<double>(), trial_xi.as<double>(), w.as<double>()};
+    r.order = order;
+    r.dir_offset = dir_offset.as<int>();
+    r.coef = coef.as<double>();
+    r.rho = rho.as<double>();
+    for (int h = 0; h < 2; ++h)
+      for (int i = 0; i < 4; ++i) r.weights[h][i] = weights[h][i].as<double>();
+    r.share = share.as<double>();
+    r.raw = raw.as<double>();
+    r.roles = roles.as<int>();
+    for (int h = 0; h < 2; ++h) r.cell_series[h] = cell_series[h].as<double>();
+    r.host_series = series;
+    return r;
+  }
 };
 std::mutex g_rules_mu;
 std::map<std::tuple<int, int, bool>, std::unique_ptr<DeviceRules>> g_rules;
@@ -84,6 +102,36 @@ const DeviceRules& device_rules(int device, int order, bool quads = false) {
     r->trial_xi.upload(sxi);
     r->w.upload(w);
     r->total = static_cast<int>(w.size());
+    r->order = order;
+    if (!quads) {
+      std::vector<int> doff{0};
+      std::vector<int> roles;
+      std::vector<double> coef, rho, share, raw, wt[2][4];
+      for (size_t c = 0; c < ncfg; ++c) {
+        const DirectionRule d = direction_rule(static_cast<int>(c), order);
+        coef.insert(coef.end(), d.coef.begin(), d.coef.end());
+        doff.push_back(static_cast<int>(coef.size() / 4));
+        for (int h = 0; h < 2; ++h)
+          for (int i = 0; i < 4; ++i)
+            wt[h][i].insert(wt[h][i].end(), d.weights[h][i].begin(), d.weights[h][i].end());
+        share.insert(share.end(), d.share.begin(), d.share.end());
+        raw.insert(raw.end(), d.raw.begin(), d.raw.end());
+        roles.push_back(d.roles);
+        if (c == 27)
+          for (int h = 0; h < 2; ++h) r->cell_series[h].upload(d.cell_series[h]);
+        // the radii of the three kinds (vertex, edge and identical configurations)
+        if (c == 0 || c == 9 || c == 27) rho.insert(rho.end(), d.rho.begin(), d.rho.end());
+      }
+      r->dir_offset.upload(doff);
+      r->coef.upload(coef);
+      r->rho.upload(rho);
+      for (int h = 0; h < 2; ++h)
+        for (int i = 0; i < 4; ++i) r->weights[h][i].upload(wt[h][i]);
+      r->share.upload(share);
+      r->raw.upload(raw);
+      r->roles.upload(roles);
+      for (int h = 0; h < 2; ++h) r->series[h] = series_rules(order, h);
+    }
     slot = std::move(r);
   }
   return *slot;
@@ -376,8 +424,7 @@ void assemble_quad_device(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& test, vo
   if (!empty && same_grid) {
     SingularPairList& pl = grid_pairs(*test.grid, device);
     const DeviceRules& dr = device_rules(device, order, true);
-    g.rules = SingularRules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                            dr.w.as<double>()};
+    g.rules = dr.view();
     g.pairs = SingularPairs{static_cast<int>(pl.test_cell.size()), pl.d_test.as<int>(),
                             pl.d_trial.as<int>(), pl.d_config.as<int>()};
     g.singular = true;
@@ -491,8 +538,7 @@ void assemble_device(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& test, void* d
     if (pairs_ready) return;
     SingularPairList& pl = grid_pairs(*test.grid, device);
     const DeviceRules& dr = device_rules(device, order);
-    rules = SingularRules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                            dr.w.as<double>()};
+    rules = dr.view();
     pairs = SingularPairs{static_cast<int>(pl.test_cell.size()), pl.d_test.as<int>(),
                           pl.d_trial.as<int>(), pl.d_config.as<int>()};
     pairs_ready = true;
@@ -689,8 +735,7 @@ SingularPairList& sweep_pairs(GridT& g, int device) { return grid_pairs(g, devic
 
 SingularRules sweep_rules(int device, int order) {
   const DeviceRules& dr = device_rules(device, order);
-  return SingularRules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                       dr.w.as<double>()};
+  return dr.view();
 }
 
 void helmholtz_sl_gradient_device(GridT& g, const Options& opts, double k, const double* d_lam,
@@ -707,8 +752,7 @@ void helmholtz_sl_gradient_device(GridT& g, const Options& opts, double k, const
   const GridGeometry& geo = grid_geometry(g, device, rule, stream, launches);
   SingularPairList& pl = grid_pairs(g, device);
   const DeviceRules& dr = device_rules(device, static_cast<int>(sit->second));
-  SingularRules rules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                      dr.w.as<double>()};
+  const SingularRules rules = dr.view();
   SingularPairs pairs{static_cast<int>(pl.test_cell.size()), pl.d_test.as<int>(),
                       pl.d_trial.as<int>(), pl.d_config.as<int>()};
   {
@@ -757,8 +801,7 @@ MatrixT* assemble_singular_csr(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& tes
     g.test_dofs = test.d_dofs.as<int>();
     g.trial_dofs = trial.d_dofs.as<int>();
     g.rule = qrule;
-    g.rules = SingularRules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                            dr.w.as<double>()};
+    g.rules = dr.view();
     g.pairs = SingularPairs{np, pl.d_test.as<int>(), pl.d_trial.as<int>(), pl.d_config.as<int>()};
     g.singular = true;
     g.same_grid = 1;
@@ -780,8 +823,7 @@ MatrixT* assemble_singular_csr(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& tes
     const DeviceRules& dr = device_rules(device, static_cast<int>(sit->second));
     np = static_cast<int>(pl.test_cell.size());
     a.pair_values.alloc(sizeof(double) * std::max(1, np * nvals));
-    SingularRules rules{dr.offset.as<int>(), dr.test_xi.as<double>(), dr.trial_xi.as<double>(),
-                        dr.w.as<double>()};
+    const SingularRules rules = dr.view();
     SingularPairs pairs{np, pl.d_test.as<int>(), pl.d_trial.as<int>(), pl.d_config.as<int>()};
     SingularArgs sa{a.kernel, a.op, a.k, cplx ? kOutC128 : kOutF64, 0, nullptr, 0,
                     a.pair_values.as<double>()};

@@ -119,6 +119,16 @@ struct DuffyRule {
   std::vector<double> test_xi, trial_xi, w;
 };
 DuffyRule duffy_rule(int config, int order);
+// The same rule as directions x radii: SingularRules::coef, rho, weights, share, raw, roles
+// and (one cell) cell_series of one configuration.
+struct DirectionRule {
+  std::vector<double> coef, rho, share, raw;
+  std::vector<double> weights[2][4], cell_series[2];
+  int roles = 0;
+};
+DirectionRule direction_rule(int config, int order);
+// The series of the inner sums of order-n rules, kernels of order rho^-1 (h = 0) or rho^-2.
+SeriesRules series_rules(int order, int h);
 // Quadrilaterals: the n x n Gauss tensor rule for a request of `npoints` (n the smallest
 // with n^2 >= npoints), the 49 vertex pairings of two quadrilaterals that share a vertex
 // (16 vertex, 32 edge, 1 identical) and their Duffy rules of 1-D order n.

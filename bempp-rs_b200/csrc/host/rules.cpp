@@ -16,6 +16,7 @@
 // mapped onto the cells' local vertices so that the shared vertex is P0 and the shared
 // edge is P0-P1 in both cells.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <functional>
 #include <stdexcept>
@@ -177,13 +178,14 @@ void to_reference(double x1, double x2, const int perm[3], double& u, double& v)
 
 }  // namespace
 
-DuffyRule duffy_rule(int config, int order) {
+namespace {
+// Local vertices that play P0, P1, P2 in the test and the trial cell of a configuration;
+// returns the number of shared vertices.
+int configuration_roles(int config, int tp[3], int sp[3]) {
   const auto& cfgs = singular_configurations();
   if (config < 0 || config >= static_cast<int>(cfgs.size()))
     throw Error(kInvalidArgument, "bad singular configuration");
-  if (order < 1) throw Error(kInvalidArgument, "singular quadrature order must be >= 1");
   const auto& pairs = cfgs[config];
-  int tp[3], sp[3];
   const int shared = static_cast<int>(pairs.size());
   auto fill_rest = [](int* perm, int used) {
     int k = used;
@@ -203,6 +205,42 @@ DuffyRule duffy_rule(int config, int order) {
     fill_rest(tp, shared);
     fill_rest(sp, shared);
   }
+  return shared;
+}
+
+// Weight of the inner coordinates (xi), (xi, a) or (xi, a, b) number j (the last fastest):
+// Gauss weights times xi^3, xi^3 a^2 or xi^3 a^2 b; the rest of a point's weight belongs to its
+// direction.
+double inner_weights(int shared, int order, int j) {
+  std::vector<double> gx, gw;
+  gauss_legendre_01(order, gx, gw);
+  double w = 1.0;
+  for (int i = shared - 1; i >= 0; --i, j /= order) {
+    const double x = gx[j % order];
+    w *= gw[j % order] * (i == 0 ? x * x * x : i == 1 ? x * x : x);
+  }
+  return w;
+}
+
+// Coefficient of (i x)^m in e^{ix} (h = 0) or (1 - ix) e^{ix} (h = 1), without the i that the
+// odd ones keep: e^{ix} = sum (ix)^m / m!, (1 - ix) e^{ix} = sum (1 - m) (ix)^m / m!.
+double phase_coefficient(int m, int h) {
+  double c = (m / 2) % 2 ? -1.0 : 1.0;
+  for (int i = 2; i <= m; ++i) c /= i;
+  return h == 0 ? c : c * (1.0 - m);
+}
+
+RegionPoint region_point(int shared, int reg, double xi, double a, double b, double c) {
+  return shared == 3   ? identical_region(reg, xi, a, b, c)
+         : shared == 2 ? edge_region(reg, xi, a, b, c)
+                       : vertex_region(reg, xi, a, b, c);
+}
+}  // namespace
+
+DuffyRule duffy_rule(int config, int order) {
+  int tp[3], sp[3];
+  const int shared = configuration_roles(config, tp, sp);
+  if (order < 1) throw Error(kInvalidArgument, "singular quadrature order must be >= 1");
   std::vector<double> gx, gw;
   gauss_legendre_01(order, gx, gw);
   const int nreg = shared == 3 ? 6 : (shared == 2 ? 5 : 2);
@@ -216,10 +254,7 @@ DuffyRule duffy_rule(int config, int order) {
       for (int i1 = 0; i1 < order; ++i1)
         for (int i2 = 0; i2 < order; ++i2)
           for (int i3 = 0; i3 < order; ++i3) {
-            const double xi = gx[i0], a = gx[i1], b = gx[i2], c = gx[i3];
-            RegionPoint p = shared == 3   ? identical_region(reg, xi, a, b, c)
-                            : shared == 2 ? edge_region(reg, xi, a, b, c)
-                                          : vertex_region(reg, xi, a, b, c);
+            const RegionPoint p = region_point(shared, reg, gx[i0], gx[i1], gx[i2], gx[i3]);
             double u, v;
             to_reference(p.x1, p.x2, tp, u, v);
             r.test_xi.push_back(u);
@@ -230,6 +265,133 @@ DuffyRule duffy_rule(int config, int order) {
             r.w.push_back(gw[i0] * gw[i1] * gw[i2] * gw[i3] * p.jac);
           }
   return r;
+}
+
+DirectionRule direction_rule(int config, int order) {
+  int tp[3], sp[3];
+  const int shared = configuration_roles(config, tp, sp);
+  const DuffyRule d = duffy_rule(config, order);
+  std::vector<double> gx, gw;
+  gauss_legendre_01(order, gx, gw);
+  const int nreg = shared == 3 ? 6 : (shared == 2 ? 5 : 2);
+  // the last 3, 2 or 1 of the cube's coordinates (xi, a, b, c) are the direction's, the
+  // product of the others is the radius
+  const int nrad = shared;
+  int per = 1, inner = 1;
+  for (int i = 0; i < 4; ++i) (i < nrad ? inner : per) *= order;
+  auto coordinates = [&](int index, int first, int count, double x[4]) {
+    for (int i = first + count - 1; i >= first; --i) {
+      x[i] = gx[index % order];
+      index /= order;
+    }
+  };
+  DirectionRule r;
+  for (int j = 0; j < inner; ++j) {
+    double x[4] = {1.0, 1.0, 1.0, 1.0};
+    coordinates(j, 0, nrad, x);
+    const double rho = x[0] * x[1] * x[2];
+    r.rho.push_back(rho);
+    r.rho.push_back(1.0 / rho);
+  }
+  // offsets x1 (P1 - P0) + x2 (P2 - P1) along the reference axes of a cell
+  auto along = [](double x1, double x2, const int perm[3], double out[2]) {
+    for (int axis = 0; axis < 2; ++axis) {
+      const double p0 = perm[0] == axis + 1, p1 = perm[1] == axis + 1, p2 = perm[2] == axis + 1;
+      out[axis] = x1 * (p1 - p0) + x2 * (p2 - p1);
+    }
+  };
+  for (int reg = 0; reg < nreg; ++reg)
+    for (int i = 0; i < per; ++i) {
+      double x[4] = {1.0, 1.0, 1.0, 1.0};
+      coordinates(i, nrad, 4 - nrad, x);
+      RegionPoint p = region_point(shared, reg, x[0], x[1], x[2], x[3]);
+      if (shared >= 2) {  // P1 - P0 is one vector in both cells
+        p.x1 -= p.y1;
+        p.y1 = 0.0;
+      }
+      if (shared == 3) {
+        p.x2 -= p.y2;
+        p.y2 = 0.0;
+      }
+      double cx[2], cy[2];
+      along(p.x1, p.x2, tp, cx);
+      along(p.y1, p.y2, sp, cy);
+      r.coef.insert(r.coef.end(), {cx[0], cx[1], cy[0], cy[1]});
+      const size_t first = static_cast<size_t>(reg) * per * inner + i;
+      r.share.push_back(d.w[first] / inner_weights(shared, order, 0));
+      const RegionPoint q = region_point(shared, reg, x[0], x[1], x[2], x[3]);
+      if (shared == 2)
+        r.raw.insert(r.raw.end(), {1.0 - q.x1, q.x2, 1.0 - q.y1, q.y2});
+      else
+        r.raw.insert(r.raw.end(), {q.x1, q.x2, q.y1, q.y2});
+      for (int h = 0; h < 2; ++h) {
+        // moments m: sums over the radii of w rho^(m - 1 - h) times the basis products;
+        // moment 0 serves the homogeneous (Laplace) kernels
+        const int rows = shared == 3 ? 2 * kSeriesTerms : 1;
+        double moment[2 * kSeriesTerms][9] = {}, total = 0.0, by_trial[4] = {}, by_test[4] = {};
+        for (int j = 0; j < inner; ++j) {
+          const size_t at = first + static_cast<size_t>(j) * per;
+          const double inv = r.rho[2 * j + 1];
+          const double u = d.test_xi[2 * at], v = d.test_xi[2 * at + 1];
+          const double s = d.trial_xi[2 * at], t = d.trial_xi[2 * at + 1];
+          const double phi[3] = {1.0 - u - v, u, v}, psi[3] = {1.0 - s - t, s, t};
+          double w = d.w[at] * (h == 0 ? inv : inv * inv);
+          total += w;
+          for (int a = 0; a < 3; ++a) {
+            by_test[a] += w * phi[a];
+            by_trial[a] += w * psi[a];
+          }
+          for (int m = 0; m < rows; ++m, w *= r.rho[2 * j])
+            for (int e = 0; e < 9; ++e) moment[m][e] += w * phi[e / 3] * psi[e % 3];
+        }
+        r.weights[h][0].push_back(total);
+        r.weights[h][1].insert(r.weights[h][1].end(), by_trial, by_trial + 4);
+        r.weights[h][2].insert(r.weights[h][2].end(), by_test, by_test + 4);
+        r.weights[h][3].insert(r.weights[h][3].end(), moment[0], moment[0] + 9);
+        r.weights[h][3].push_back(0.0);
+        if (rows == 1) continue;
+        for (int m = 0; m < rows; ++m) {
+          const double c = phase_coefficient(m, h);
+          for (int e = 0; e < 9; ++e) r.cell_series[h].push_back(c * moment[m][e]);
+          r.cell_series[h].push_back(0.0);
+        }
+      }
+    }
+  for (int v = 0; v < 3; ++v) r.roles |= (tp[v] << (2 * v)) | (sp[v] << (6 + 2 * v));
+  return r;
+}
+
+SeriesRules series_rules(int order, int h) {
+  SeriesRules out{};
+  std::vector<double> gx, gw;
+  gauss_legendre_01(order, gx, gw);
+  auto put = [&](int q, int shared, const std::function<double(double, double)>& mu) {
+    int inner = 1;
+    for (int i = 0; i < shared; ++i) inner *= order;
+    double sum[2 * kSeriesTerms] = {};
+    for (int j = 0; j < inner; ++j) {
+      // inner coordinates (xi), (xi, a) or (xi, a, b), the last fastest; radius: their product
+      double rho = 1.0, xi = 1.0;
+      for (int i = 0, rest = j; i < shared; ++i, rest /= order) {
+        rho *= gx[rest % order];
+        xi = gx[rest % order];  // the last one taken is the first coordinate
+      }
+      double w = inner_weights(shared, order, j) * mu(xi, rho) / (h == 0 ? rho : rho * rho);
+      for (int m = 0; m < 2 * kSeriesTerms; ++m, w *= rho) sum[m] += w;
+    }
+    for (int m = 0; m < 2 * kSeriesTerms; ++m) out.c[q][m] = phase_coefficient(m, h) * sum[m];
+  };
+  put(0, 1, [](double, double) { return 1.0; });
+  put(1, 1, [](double xi, double) { return xi; });
+  put(2, 1, [](double xi, double) { return xi * xi; });
+  put(3, 2, [](double, double) { return 1.0; });
+  put(4, 2, [](double xi, double) { return xi; });
+  put(5, 2, [](double, double rho) { return rho; });
+  put(6, 2, [](double xi, double) { return xi * xi; });
+  put(7, 2, [](double xi, double rho) { return xi * rho; });
+  put(8, 2, [](double, double rho) { return rho * rho; });
+  put(9, 3, [](double, double) { return 1.0; });
+  return out;
 }
 
 // ------------------------------------------------------------------ quadrilaterals ---

@@ -105,12 +105,42 @@ cudaError_t launch_regular_fp64(const CellSet& test, const SpaceTiles& tt, const
                                 const SpaceTiles& st, const RegularRule& rule,
                                 const RegularArgs& a, cudaStream_t stream, bool direct);
 
+// Power series of the inner sums of the Duffy rules (singular.cu): P_q(theta) = sum_n z^n
+// (c[q][2n] + i theta c[q][2n + 1]), z = theta^2; q 0 .. 2: common vertex, inner basis products
+// 1, xi, xi^2; 3 .. 8: edge, 1, xi, rho, xi^2, xi rho, rho^2; 9: one cell, 1.
+constexpr int kSeriesTerms = 16;
+struct SeriesRules {
+  double c[10][2 * kSeriesTerms];
+};
+
 // Singular (Duffy) rules of all 28 adjacency configurations, concatenated.
 struct SingularRules {
   const int* offset;       // 29 entries: first point of each configuration
   const double* test_xi;   // 2 * total
   const double* trial_xi;  // 2 * total
   const double* w;         // total
+  // Triangles: the same rules as products of directions and radii (see singular.cu).
+  // Point (region, i) x j of a configuration is point region n^4 + j per + i above, per the
+  // number of directions of a region (n^3, n^2, n for a common vertex, edge, cell).
+  int order = 0;                      // n
+  const int* dir_offset = nullptr;    // 29 entries: first direction of each configuration
+  const double* coef = nullptr;       // 4 per direction: d = c0 t0x + c1 t1x - c2 t0y - c3 t1y
+  const double* rho = nullptr;        // (rho, 1/rho) of the n, n^2, n^3 radii of the three kinds
+  // sums over the radii of w rho^-1 (first index 0) or w rho^-2 (1) times the basis
+  // products, per direction: total; by trial basis (3 of 4); by test basis (3 of 4); by
+  // both (9 of 10, test basis first)
+  const double* weights[2][4] = {};
+  // Helmholtz: the share of the weights that belongs to a direction, its raw coordinates
+  // (common vertex: x1, x2, y1, y2 = xi times these; edge: x1 = xi - X1 rho, x2 = X2 rho,
+  // the same for y), the local vertices that play P0, P1, P2 (two bits each, test cell
+  // first; 28 entries), the block's series per direction of the one-cell configuration
+  // (first index as weights; kSeriesTerms pairs of rows of 10 values), and the series of the
+  // inner sums (two, as weights; host memory, passed to the kernel as constants)
+  const double* share = nullptr;
+  const double* raw = nullptr;
+  const int* roles = nullptr;
+  const double* cell_series[2] = {};
+  const SeriesRules* host_series = nullptr;
 };
 
 // Adjacent cell pairs (test cell, trial cell, configuration), grouped by configuration.
