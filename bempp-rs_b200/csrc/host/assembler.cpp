@@ -704,8 +704,8 @@ void assemble_potential_device(BoundaryAssemblerT& a, SpaceT& space, const doubl
     ++a.launches;
   }
   BEMPP_CUDA(launch_potential(a.kernel, a.op, d_points, static_cast<int>(npoints),
-                              cell_set(*space.grid, geo), space.d_dofs.as<int>(), space.nbasis,
-                              rule, a.k, static_cast<double*>(out), npoints, stream));
+                              cell_set(*space.grid, geo), space_tiles(space), rule, a.k,
+                              static_cast<double*>(out), npoints, stream));
   ++a.launches;
   if (single) {
     BEMPP_CUDA(launch_convert_to_single(static_cast<const double*>(out), d_out, reals, stream));
