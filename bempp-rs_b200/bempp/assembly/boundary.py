@@ -114,7 +114,8 @@ def _host_output(shape, dtype):
     Large matrices live in page-locked blocks of the library's cache: the library then
     writes the finished columns into them by DMA while later columns are still being
     computed, with no staging copy, and a block freed by one result is reused by the
-    next.  Every entry is overwritten by the assembly.
+    next.  Every entry is overwritten by the assembly, so pageable memory is not cleared
+    first (its pages are touched by the library's copy threads, while the GPU works).
     """
     nbytes = int(np.prod(shape)) * np.dtype(dtype).itemsize
     if PINNED_OUTPUT_MIN_BYTES is not None and nbytes >= PINNED_OUTPUT_MIN_BYTES:
@@ -122,7 +123,7 @@ def _host_output(shape, dtype):
             return np.asarray(_PageLockedBlock(shape, dtype))
         except MemoryError:  # page-locking refused: pageable memory
             pass
-    return np.zeros(shape, dtype=dtype, order="F")
+    return np.empty(shape, dtype=dtype, order="F")
 
 
 class BoundaryAssemblerOptions(object):
