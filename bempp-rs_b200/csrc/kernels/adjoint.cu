@@ -17,14 +17,13 @@
 // registers and shared memory, trial side by warp shuffles) and added per cell, then a
 // last kernel scatters the per-cell-vertex gradients to the vertices.
 //
-// Regular pairs use the tiled mapping of regular.cu (32 x 32 cell tiles, lane = test
-// cell, both tiles staged in shared memory by TMA bulk copies on an mbarrier with the
-// regular kernels' bounded wait and timeout counter); adjacent pairs use one warp per pair
-// over their Duffy rule.  FP64, or mixed:
+// Regular pairs use 32 x 32 cell tiles (lane = test cell, both tiles staged in shared memory
+// by TMA bulk copies on an mbarrier with the regular kernels' bounded wait and timeout
+// counter); adjacent pairs use one warp per pair over their Duffy rule.  FP64 with the
+// 6-point rule: adjoint_sl_orbits.  Other rules in FP64: adjoint_sl_regular.  Mixed:
 // far pairs (centroid distance >= 2 diameters) in FP32 with centroid-relative points and
 // the reference phase e^{ik r0} folded into the pair weight, as in regular.cu.
-#include "launch.h"
-#include "tiles.cuh"
+#include "regular_fp64.cuh"
 
 namespace bempp_b200 {
 namespace {
@@ -347,6 +346,317 @@ __global__ void __launch_bounds__(kThreads, 3)
   }
 }
 
+// The regular pairs in FP64 with the 6-point rule, on the distances and kernel values of
+// regular_fp64.cuh (registers only, two operations per squared distance).  With
+// x_p = c + gamma_p g_a, y_q = c' + gamma_q g'_b and the scalars
+//   h_pq = Re(c e^{ikr} (ikr - 1)) / r^3,
+// every vector sum of h_pq (x_p - y_q) is a combination of dc and the g's with scalar
+// coefficients: row sums R_p = sum_q w_q h_pq, column sums, and G_pb = sum over the trial
+// orbits of w gamma h.  So the loop over point pairs keeps scalars (about 5 operations per
+// pair for all sums, where accumulating the vectors per test and per trial point took 8 and
+// the differences 3 more) and the vectors are formed once per cell pair.
+// The largest circumradii of the two tiles decide between the phase referenced to the pair and
+// the reduced phase.  5,120 triangles, k = 5, B200: 3.3 ms with coordinate differences,
+// 1.97 in this form.
+template <int PH>
+__device__ __forceinline__ void adjoint_orbit_pairs(
+    const Tile& T, const Tile& S, int it, int warp, int ti0, int sj0, int nti, int nsj, bool both,
+    const fp64::OrbitRule& rule, double k, const double2* __restrict__ lam,
+    const double2* __restrict__ mu, const double* jx, const double* jy, double* s_test,
+    double* s_trial, double& jval, double& dk) {
+  using namespace fp64;
+  const bool valid = it < nti;
+  const double2 li = valid ? lam[ti0 + it] : make_double2(0.0, 0.0);
+  const double2 mi = valid && both ? mu[ti0 + it] : make_double2(0.0, 0.0);
+  const int a0 = T.vid[it], a1 = T.vid[kTile + it], a2 = T.vid[2 * kTile + it];
+  double* mine = s_test + warp * 9 * kTile + it;
+#pragma unroll 1
+  for (int js = warp; js < nsj; js += kWarps) {
+    const bool active = valid && !share_vertex(a0, a1, a2, S.vid[js], S.vid[kTile + js],
+                                               S.vid[2 * kTile + js]);
+    // c = conj(lambda_i) mu_j (+ conj(lambda_j) mu_i off the diagonal)
+    const double2 mj = mu[sj0 + js];
+    double c_re = li.x * mj.x + li.y * mj.y, c_im = li.x * mj.y - li.y * mj.x;
+    if (both) {
+      const double2 lj = lam[sj0 + js];
+      c_re += lj.x * mi.x + lj.y * mi.y;
+      c_im += lj.x * mi.y - lj.y * mi.x;
+    }
+    PairGeometry p;
+    pair_geometry<kHelmholtz, kSL, 1, 1, false>(T, it, S, js, 1.0, p);
+    // phase referenced to the pair: c is rotated by e^{ik r0} for the gradient terms, the
+    // sums S0, Sk after the loop
+    double kr0 = 0.0, pc = 1.0, ps = 0.0, q_re = c_re, q_im = c_im;
+    if (PH == kReferenced) {
+      kr0 = k * (p.r0 * rsqrt_refined(p.r0));
+      sincos_any(kr0, ps, pc);
+      q_re = c_re * pc - c_im * ps;
+      q_im = c_re * ps + c_im * pc;
+    }
+    double M[3][3], Y[2][3];
+    M[0][0] = p.m00;
+    M[0][1] = p.m01;
+    M[1][0] = p.m10;
+    M[1][1] = p.m11;
+    M[0][2] = -(p.m00 + p.m01);
+    M[1][2] = -(p.m10 + p.m11);
+    M[2][0] = -(p.m00 + p.m10);
+    M[2][1] = -(p.m01 + p.m11);
+    M[2][2] = -(M[2][0] + M[2][1]);
+    const double dgx[3] = {p.dgx0, p.dgx1, -(p.dgx0 + p.dgx1)};
+    const double dgy[3] = {p.dgy0, p.dgy1, -(p.dgy0 + p.dgy1)};
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const double e = S.G(rE + b, js);
+#pragma unroll
+      for (int o = 0; o < 2; ++o) Y[o][b] = fma(rule.g2[o], e, -2.0 * rule.g[o] * dgy[b]);
+    }
+    double S0_re = 0.0, S0_im = 0.0, Sk_re = 0.0, Sk_im = 0.0;
+    // sums of h: columns (times the test weight), w phi_a w gamma by (test, trial vertex),
+    // and the row sums' combinations
+    double col[2][3] = {{0, 0, 0}, {0, 0, 0}}, Cd[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    double cC[3] = {0, 0, 0}, Db[3] = {0, 0, 0}, Ad[3] = {0, 0, 0}, cA = 0.0;
+    double BR[3] = {0, 0, 0}, BD[3] = {0, 0, 0};
+#pragma unroll 1
+    for (int op = 0; op < 2; ++op) {
+      const double gp = rule.g[op], g2 = rule.g2[op], wp = rule.w[op], cp = rule.c[op],
+                   dp = rule.d[op], m0 = rule.m[op][0], m1 = rule.m[op][1];
+      double s0r[2] = {0, 0}, s0i[2] = {0, 0}, skr[2] = {0, 0}, ski[2] = {0, 0};
+      double sumG[3] = {0, 0, 0}, sumR = 0.0;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double X = fma(g2, T.G(rE + a, it), fma(2.0 * gp, dgx[a], p.r0));
+        double h[6];
+        {
+          double r2[6], y[6], t[6], kr[6], sn[6], csn[6];
+#pragma unroll
+          for (int i = 0; i < 6; ++i) r2[i] = X + Y[i / 3][i % 3];
+#pragma unroll
+          for (int i = 0; i < 6; ++i) r2[i] = fma(i < 3 ? m0 : m1, M[a][i % 3], r2[i]);
+#pragma unroll
+          for (int i = 0; i < 6; ++i) y[i] = rsqrt_refined(r2[i]);
+#pragma unroll
+          for (int i = 0; i < 6; ++i) kr[i] = k * (r2[i] * y[i]);
+          if (PH == kReferenced) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) t[i] = kr[i] - kr0;
+            sincos_small_n<6>(t, sn, csn);
+          } else {
+            sincos_any_n<6>(kr, sn, csn);
+          }
+#pragma unroll
+          for (int i = 0; i < 6; ++i) {
+            s0r[i / 3] = fma(y[i], csn[i], s0r[i / 3]);
+            s0i[i / 3] = fma(y[i], sn[i], s0i[i / 3]);
+            skr[i / 3] += csn[i];
+            ski[i / 3] += sn[i];
+          }
+          // Re(q e^{ikr} (ikr - 1)) / r^3
+#pragma unroll
+          for (int i = 0; i < 6; ++i) {
+            const double fr = fma(kr[i], sn[i], csn[i]), fi = fma(kr[i], csn[i], -sn[i]);
+            h[i] = -(fma(q_im, fi, q_re * fr)) * (y[i] * y[i] * y[i]);
+          }
+        }
+        const double sum0 = (h[0] + h[1]) + h[2], sum1 = (h[3] + h[4]) + h[5];
+        const double R = fma(rule.w[1], sum1, rule.w[0] * sum0);
+        const double base = fma(rule.c[1], sum1, rule.c[0] * sum0);
+        sumR += R;
+        Ad[a] = fma(dp, R, Ad[a]);
+        BR[a] = fma(gp * cp, R, BR[a]);
+        BD[a] = fma(gp * dp, R, BD[a]);
+        Db[a] = fma(dp, base, Db[a]);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          const double G = fma(rule.d[1], h[3 + b], rule.d[0] * h[b]);
+          Cd[a][b] = fma(dp, G, Cd[a][b]);
+          sumG[b] += G;
+          col[0][b] = fma(wp, h[b], col[0][b]);
+          col[1][b] = fma(wp, h[3 + b], col[1][b]);
+        }
+      }
+      cA = fma(cp, sumR, cA);
+#pragma unroll
+      for (int b = 0; b < 3; ++b) cC[b] = fma(cp, sumG[b], cC[b]);
+      S0_re = fma(wp, fma(rule.w[1], s0r[1], rule.w[0] * s0r[0]), S0_re);
+      S0_im = fma(wp, fma(rule.w[1], s0i[1], rule.w[0] * s0i[0]), S0_im);
+      Sk_re = fma(wp, fma(rule.w[1], skr[1], rule.w[0] * skr[0]), Sk_re);
+      Sk_im = fma(wp, fma(rule.w[1], ski[1], rule.w[0] * ski[0]), Sk_im);
+    }
+    if (PH == kReferenced) {
+      const double s0r = S0_re * pc - S0_im * ps, s0i = S0_re * ps + S0_im * pc;
+      const double skr = Sk_re * pc - Sk_im * ps, ski = Sk_re * ps + Sk_im * pc;
+      S0_re = s0r;
+      S0_im = s0i;
+      Sk_re = skr;
+      Sk_im = ski;
+    }
+    const double jdet_i = T.G(rJ, it), jdet_j = S.G(rJ, js);
+    const double jj = jdet_i * jdet_j * kInv4Pi;
+    const double R0 = c_re * S0_re - c_im * S0_im;  // Re(c S0)
+    const double ri = R0 * jdet_j * kInv4Pi, rj = R0 * jdet_i * kInv4Pi;
+    // column combinations of the trial side: w phi_b and w phi_b gamma
+    const double k0 = (col[0][0] + col[0][1]) + col[0][2], k1 = (col[1][0] + col[1][1]) + col[1][2];
+    const double cB = fma(rule.c[1], k1, rule.c[0] * k0);
+    double Bd[3], Tb[3], Td[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      Bd[b] = cB + fma(rule.d[1], col[1][b], rule.d[0] * col[0][b]);
+      Tb[b] = fma(rule.g[1] * rule.c[1], col[1][b], rule.g[0] * rule.c[0] * col[0][b]);
+      Td[b] = fma(rule.g[1] * rule.d[1], col[1][b], rule.g[0] * rule.d[0] * col[0][b]);
+    }
+    double gs[9];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double dc = (T.G(rC + d, it) - S.G(rC + d, js)) + (T.G(rL + d, it) - S.G(rL + d, js));
+      const double gx0 = T.G(rG0 + d, it), gx1 = T.G(rG1 + d, it), gy0 = S.G(rG0 + d, js), gy1 = S.G(rG1 + d, js);
+      const double gx[3] = {gx0, gx1, -(gx0 + gx1)}, gy[3] = {gy0, gy1, -(gy0 + gy1)};
+      const double vx = fma(gx0, BR[0] - BR[2], gx1 * (BR[1] - BR[2]));
+      const double vy = fma(gy0, Tb[0] - Tb[2], gy1 * (Tb[1] - Tb[2]));
+      // sum over q of the trial offsets with the c-part of the test basis
+      const double wc = fma(gy0, cC[0] - cC[2], gy1 * (cC[1] - cC[2]));
+      const double wb = fma(gx0, Db[0] - Db[2], gx1 * (Db[1] - Db[2]));
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double C = fma(gy0, Cd[a][0] - Cd[a][2], gy1 * (Cd[a][1] - Cd[a][2]));
+        const double vt = fma(dc, cA + Ad[a], vx) + fma(gx[a], BD[a], -(wc + C));
+        if (active) mine[(3 * a + d) * kTile] += fma(jj, vt, ri * jx[(3 * a + d) * kTile + it]);
+        const double D = fma(gx0, Cd[0][a] - Cd[2][a], gx1 * (Cd[1][a] - Cd[2][a]));
+        const double ut = fma(dc, Bd[a], wb + D) - fma(gy[a], Td[a], vy);
+        gs[3 * a + d] = active ? fma(-jj, ut, rj * jy[(3 * a + d) * kTile + js]) : 0.0;
+      }
+    }
+    if (active) {
+      jval = fma(R0, jj, jval);
+      dk += (c_re * (-Sk_im) - c_im * Sk_re) * jj;  // Re(c i Sk)
+    }
+    // trial side: nine sums over the lanes; eight of them by halves (lane l ends with value
+    // l / 4), 14 exchanges in place of 45
+    double v4[4], v2[2], v1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool hi = it & 16;
+      v4[i] = (hi ? gs[i + 4] : gs[i]) + __shfl_xor_sync(0xffffffffu, hi ? gs[i] : gs[i + 4], 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const bool hi = it & 8;
+      v2[i] = (hi ? v4[i + 2] : v4[i]) + __shfl_xor_sync(0xffffffffu, hi ? v4[i] : v4[i + 2], 8);
+    }
+    {
+      const bool hi = it & 4;
+      v1 = (hi ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, hi ? v2[0] : v2[1], 4);
+    }
+    v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
+    v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
+    double v8 = gs[8];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) v8 += __shfl_xor_sync(0xffffffffu, v8, s);
+    if ((it & 3) == 0) s_trial[js * 9 + (it >> 2)] += v1;  // each js belongs to one warp
+    if (it == 1) s_trial[js * 9 + 8] += v8;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    adjoint_sl_orbits(CellSet cs, const __grid_constant__ fp64::OrbitRule rule, double k,
+                      const double2* __restrict__ lam, const double2* __restrict__ mu,
+                      double* __restrict__ grad_cell, double* __restrict__ totals,
+                      unsigned* __restrict__ stage_timeouts, int stage_polls) {
+  using namespace fp64;
+  int tx, sy;
+  const int ntt = (cs.ncells + kTile - 1) / kTile;
+  lower_tile_pair(blockIdx.x, ntt, 0, ntt, tx, sy);
+  const bool both = tx > sy;
+  const int ti0 = tx * kTile, sj0 = sy * kTile;
+  const int nti = min(kTile, cs.ncells - ti0), nsj = min(kTile, cs.ncells - sj0);
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);  // completion of the tile copies
+  constexpr size_t kTileBytes = kStagedBytes;
+  const Tile T = tile_at(smem + 16), S = tile_at(smem + 16 + kTileBytes);
+  double* jx = reinterpret_cast<double*>(smem + 16 + 2 * kTileBytes);  // d jdet / d V, [e * kTile + c]
+  double* jy = jx + 9 * kTile;
+  double* s_test = jy + 9 * kTile;                   // [warp][9][kTile] test-cell gradients
+  double* s_trial = s_test + kWarps * 9 * kTile;     // [kTile][9] trial-cell gradients
+  double* s_tot = s_trial + kTile * 9;               // J, dJ/dk
+  if (threadIdx.x == 0) mbar_init(mbar, 1);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(mbar, 2 * kStagedBytes);
+    stage_geometry(T, cs, ti0, mbar);
+    stage_geometry(S, cs, sj0, mbar);
+  }
+  for (int e = threadIdx.x; e < (kWarps + 1) * kTile * 9 + 2; e += kThreads) s_test[e] = 0.0;
+  const bool staged = mbar_wait_bounded(mbar, 0, stage_polls);
+  if (__syncthreads_or(!staged)) {
+    // the copies did not complete in time: record it, give them a last bounded wait and
+    // add nothing (the host reports the failure)
+    if (threadIdx.x == 0) atomicAdd(stage_timeouts, 1u);
+    mbar_wait_bounded(mbar, 0);
+    return;
+  }
+  const int it = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // every phase k (r - r0) of the tile pair is at most k (largest rad_x + largest rad_y)
+  bool referenced;
+  {
+    double rx = it < nti ? T.G(kRad, it) : 0.0, ry = it < nsj ? S.G(kRad, it) : 0.0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      rx = fmax(rx, __shfl_xor_sync(0xffffffffu, rx, s));
+      ry = fmax(ry, __shfl_xor_sync(0xffffffffu, ry, s));
+    }
+    referenced = fabs(k) * (rx + ry) <= 0.8;
+  }
+  __syncthreads();  // the rows of kRad change meaning below
+  if (warp < 2) {
+    const Tile& t = warp == 0 ? T : S;
+    double t0[3], t1[3], n[3], dj[3][3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      t0[d] = t.G(kT0x + d, it);
+      t1[d] = t.G(kT1x + d, it);
+      n[d] = t.G(kNx + d, it);
+    }
+    jdet_gradient(t0, t1, n, dj);
+#pragma unroll
+    for (int e = 0; e < 9; ++e) (warp == 0 ? jx : jy)[e * kTile + it] = dj[e / 3][e % 3];
+    geometry_to_offsets(t, it);
+  }
+  __syncthreads();
+
+  double jval = 0.0, dk = 0.0;
+  if (referenced)
+    adjoint_orbit_pairs<kReferenced>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k, lam, mu, jx,
+                                     jy, s_test, s_trial, jval, dk);
+  else
+    adjoint_orbit_pairs<kAnyPhase>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k, lam, mu, jx,
+                                   jy, s_test, s_trial, jval, dk);
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    jval += __shfl_xor_sync(0xffffffffu, jval, s);
+    dk += __shfl_xor_sync(0xffffffffu, dk, s);
+  }
+  if (it == 0) {
+    atomicAdd(s_tot, jval);
+    atomicAdd(s_tot + 1, dk);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < kTile * 9; e += kThreads) {
+    const int c = e / 9, f = e % 9;
+    if (c < nti) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) v += s_test[(w * 9 + f) * kTile + c];
+      atomicAdd(grad_cell + static_cast<int64_t>(ti0 + c) * 9 + f, v);
+    }
+    if (c < nsj) atomicAdd(grad_cell + static_cast<int64_t>(sj0 + c) * 9 + f, s_trial[e]);
+  }
+  if (threadIdx.x == 0) {
+    atomicAdd(totals, s_tot[0]);
+    atomicAdd(totals + 1, s_tot[1]);
+  }
+}
+
 struct CellGeo {
   double v0[3], t0[3], t1[3], n[3], jdet;
 };
@@ -480,10 +790,21 @@ cudaError_t launch_adjoint_sl(const CellSet& cs, const RegularRule& rule,
   const dim3 grid(static_cast<unsigned>(ntt * (ntt + 1) / 2));  // tile pairs tx >= sy
   const double2* l2 = reinterpret_cast<const double2*>(lam);
   const double2* m2 = reinterpret_cast<const double2*>(mu);
-  auto fn = rule.npts == 6 ? (mixed ? adjoint_sl_regular<6, true> : adjoint_sl_regular<6, false>)
-                           : (mixed ? adjoint_sl_regular<0, true> : adjoint_sl_regular<0, false>);
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  fn<<<grid, kThreads, smem, stream>>>(cs, rule, k, l2, m2, grad_cell, totals, timeouts, polls);
+  if (!mixed && fp64::has_orbit_form(rule)) {
+    const size_t bytes = 16 + 2 * fp64::kStagedBytes +
+                         sizeof(double) * ((2 * 9 + (kWarps + 1) * 9) * kTile + 2);
+    e = cudaFuncSetAttribute(adjoint_sl_orbits, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(bytes));
+    if (e != cudaSuccess) return e;
+    adjoint_sl_orbits<<<grid, kThreads, bytes, stream>>>(cs, fp64::orbit_rule(rule), k, l2, m2,
+                                                         grad_cell, totals, timeouts, polls);
+  } else {
+    auto fn = rule.npts == 6 ? adjoint_sl_regular<6, true>
+              : mixed        ? adjoint_sl_regular<0, true>
+                             : adjoint_sl_regular<0, false>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    fn<<<grid, kThreads, smem, stream>>>(cs, rule, k, l2, m2, grad_cell, totals, timeouts, polls);
+  }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (pairs.npairs > 0) {
     adjoint_sl_singular<<<(pairs.npairs + 7) / 8, 256, 0, stream>>>(cs, rules, pairs, k, l2, m2,
