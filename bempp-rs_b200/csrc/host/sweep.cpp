@@ -145,11 +145,13 @@ void helmholtz_sl_sweep_device(GridT* const* grids, size_t ngrids, const double*
     a.near_begin[0] = a.sing_begin[0] = 0;
     for (size_t r = 0; r < ngrids; ++r) {
       a.near_begin[r + 1] = a.near_begin[r] + static_cast<long long>(a.mesh[r].nnear) * nk;
-      a.sing_begin[r + 1] = a.sing_begin[r] + static_cast<long long>(a.mesh[r].sing.npairs) * nk;
+      a.sing_begin[r + 1] = a.sing_begin[r] + a.mesh[r].sing.npairs;
     }
     a.ks = plan->d_ks.as<double>();
     a.nk = static_cast<int>(nk);
     a.counter = plan->d_counter.as<unsigned long long>();
+    int polls = 0;
+    BEMPP_CUDA(stage_wait_state(&a.stage_timeouts, &polls));
     const int sms = sm_count(device);
 
     // autotune once per (device, mesh sizes, nk), unless the caller fixed the parameters
@@ -179,7 +181,7 @@ void helmholtz_sl_sweep_device(GridT* const* grids, size_t ngrids, const double*
             probe.nitems = std::min<long long>(full, std::max<long long>(full / 16, 8LL * sms));
             BEMPP_CUDA(cudaMemsetAsync(probe.counter, 0, sizeof(unsigned long long), ts));
             BEMPP_CUDA(cudaEventRecord(e0, ts));
-            BEMPP_CUDA(launch_sweep_sl(probe, rule, rules, bps, sms, ts));
+            BEMPP_CUDA(launch_sweep_sl(probe, rule, bps, sms, ts));
             BEMPP_CUDA(cudaEventRecord(e1, ts));
             BEMPP_CUDA(cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -218,7 +220,7 @@ void helmholtz_sl_sweep_device(GridT* const* grids, size_t ngrids, const double*
     if (e1 == cudaSuccess) e1 = launch_sweep_near_singular(a, rule, rules, side);
     if (e1 == cudaSuccess) e1 = cudaEventRecord(join, side);
     cudaError_t e2 = e1 == cudaSuccess ? cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), cs) : e1;
-    if (e2 == cudaSuccess) e2 = launch_sweep_sl(a, rule, rules, plan->tuning.blocks_per_sm, sms, cs);
+    if (e2 == cudaSuccess) e2 = launch_sweep_sl(a, rule, plan->tuning.blocks_per_sm, sms, cs);
     if (e2 == cudaSuccess && e1 == cudaSuccess) e2 = cudaStreamWaitEvent(cs, join, 0);
     cudaError_t e3 = cudaStreamEndCapture(cs, &plan->graph);
     cudaStreamDestroy(cs);

@@ -271,7 +271,7 @@ cudaError_t launch_adjoint_sl(const CellSet& cs, const RegularRule& rule,
                               double* grad_points, int npoints, double* totals, bool mixed,
                               cudaStream_t stream);
 
-// Batched Helmholtz single-layer DP0 sweep (regular.cu): one persistent launch over
+// Batched Helmholtz single-layer DP0 sweep (sweep.cu): one persistent launch over
 // every (mesh, test tile, trial tile, wavenumber chunk) item; complex64 outputs.
 constexpr int kMaxSweepMeshes = 8;
 struct SweepMesh {
@@ -297,18 +297,18 @@ struct SweepArgs {
   int tile_shape = 1;     // a work item covers tile_shape x tile_shape pairs of 32-cell tiles
   long long nitems;
   unsigned long long* counter;  // work counter, zeroed before each launch
-  // prefix sums over the meshes of (near pairs x nk) and (vertex-sharing pairs x nk)
+  unsigned* stage_timeouts;     // counts the CTAs whose tile copies did not complete in time
+  // prefix sums over the meshes of (near pairs x nk) and of the vertex-sharing pairs
   long long near_begin[kMaxSweepMeshes + 1];
   long long sing_begin[kMaxSweepMeshes + 1];
 };
 size_t sweep_smem_bytes(int tile_shape);
 // The far pairs of every item: persistent launch of blocks_per_sm (at most 6) x sms CTAs
 // (FP32, the pairs marked in the meshes' near-field masks left alone).
-cudaError_t launch_sweep_sl(const SweepArgs& args, const RegularRule& rule,
-                            const SingularRules& rules, int blocks_per_sm, int sms,
-                            cudaStream_t stream);
+cudaError_t launch_sweep_sl(const SweepArgs& args, const RegularRule& rule, int blocks_per_sm,
+                            int sms, cudaStream_t stream);
 // The near pairs (FP64, one thread per pair and wavenumber) and the vertex-sharing pairs
-// (their Duffy rules, FP64, one warp per pair and wavenumber) of every mesh and
+// (their Duffy rules, FP64, a few threads per pair and four wavenumbers) of every mesh and
 // wavenumber: they write the entries the far-pair launch leaves alone, so both may run
 // concurrently.
 cudaError_t launch_sweep_near_singular(const SweepArgs& args, const RegularRule& rule,

@@ -1211,267 +1211,6 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ------------------------------------------------------------------------------------
-// Batched Helmholtz single-layer DP0 sweep over many wavenumbers and meshes.
-//
-// One persistent launch for the far pairs: every CTA repeatedly takes the next work item
-// (mesh, chunk of wavenumbers, super-tile pair) from a global counter (items of the
-// largest mesh first), stages the tiles once, and for each wavenumber of its chunk writes
-// the far-pair entries of its 32 x 32 blocks in FP32 (block_fp32), complex64.  The pairs
-// the mesh's near field marks (centroid distance below twice the larger diameter, or a
-// shared vertex: the same masks as the one-off mixed assembly) are left to two FP64
-// launches that run beside it (forked in the same captured graph): near pairs by the
-// 6-point rule with the pair-referenced phase, vertex-sharing pairs by their Duffy rules.
-// The single layer is symmetric on one mesh, so only tile pairs (test tile >= trial tile)
-// are items: an off-diagonal block is also written transposed (through shared memory,
-// coalesced).  No two launches or items write the same entry, so nothing orders them;
-// the only shared state is the item counter (reset before every launch).
-
-// TS: tile shape of a work item, TS x TS tiles of 32 cells on each side (a super-tile
-// pair: 1 x 1 or 2 x 2 tile pairs staged together); MINB: CTAs per SM the register
-// allocation must allow (4: up to 128 registers, 6: up to 80).  Far pairs only: the pairs
-// marked in the mesh's near-field masks (near or vertex-sharing) are written by
-// sweep_near_fp64 / sweep_duffy_fp64.
-template <int TS, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
-    sweep_sl_dp0(SweepArgs a, RegularRule rule) {
-  const int Q = 6;
-  extern __shared__ __align__(16) unsigned char smem[];
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);  // completion of the tile copies
-  unsigned char* cursor = smem + 16;
-  Tile Tt[TS], St[TS];
-#pragma unroll
-  for (int i = 0; i < TS; ++i) Tt[i] = carve_tile(cursor, Q, true, 1, false);
-#pragma unroll
-  for (int i = 0; i < TS; ++i) St[i] = carve_tile(cursor, Q, true, 1, false);
-  long long* s_item = reinterpret_cast<long long*>(cursor);
-  float2* mir = reinterpret_cast<float2*>(s_item + 2);  // [js * (kTile + 1) + it]
-  unsigned* skip = reinterpret_cast<unsigned*>(mir + kTile * (kTile + 1));  // [it]: bit js
-  const int it = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) mbar_init(mbar, 1);
-  unsigned phase = 0;  // parity of the mbarrier phase of the current item's copies
-  for (;;) {
-    if (threadIdx.x == 0) *s_item = static_cast<long long>(atomicAdd(a.counter, 1ull));
-    __syncthreads();
-    const long long item = *s_item;
-    if (item >= a.nitems) break;
-    int m = 0;
-    while (m + 1 < a.nmesh && item >= a.mesh[m + 1].item_begin) ++m;
-    const SweepMesh& M = a.mesh[m];
-    const long long local = item - M.item_begin;
-    // wavenumber chunk outermost: the items resident at one time write one output
-    // matrix (one chunk of them), in the banded order of the super-tile pairs
-    const int nsup = (M.ntiles + TS - 1) / TS;
-    const long long npairs = lower_tile_pair_count(nsup, 0, nsup);
-    const int kc = static_cast<int>(local / npairs);
-    int TT, ST;
-    lower_tile_pair(local % npairs, nsup, 0, nsup, TT, ST);
-    const int nc = M.cells.ncells;
-    // every tile of the two super-tiles by bulk (TMA) copies on the mbarrier (no FP64
-    // points: the far pairs use the FP32 offsets); the previous item's reads of the tiles
-    // ended at the barriers that closed it
-    if (threadIdx.x == 0) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      unsigned bytes = 0;
-      for (int i = 0; i < TS; ++i) {
-        if (TS * TT + i < M.ntiles) bytes += bulk_tile_bytes(Q, true, false);
-        if (TS * ST + i < M.ntiles) bytes += bulk_tile_bytes(Q, true, false);
-      }
-      mbar_expect_tx(mbar, bytes);
-      for (int i = 0; i < TS; ++i) {
-        if (TS * TT + i < M.ntiles)
-          stage_tile_bulk(Tt[i], M.cells, (TS * TT + i) * kTile, Q, true, mbar, false);
-        if (TS * ST + i < M.ntiles)
-          stage_tile_bulk(St[i], M.cells, (TS * ST + i) * kTile, Q, true, mbar, false);
-      }
-    }
-    const bool staged = mbar_wait_bounded(mbar, phase);
-    phase ^= 1u;
-    if (__syncthreads_or(!staged)) {
-      // the copies did not complete in time (never expected): record it, give them a last
-      // bounded wait and stop this CTA (the item's entries stay unwritten; the host's
-      // completion check reports it)
-      if (threadIdx.x == 0) atomicAdd(&g_stage_timeouts, 1u);
-      mbar_wait_bounded(mbar, phase ^ 1u);
-      return;
-    }
-#pragma unroll 1
-    for (int sub = 0; sub < TS * TS; ++sub) {
-      const int tt = TS * TT + sub / TS, st = TS * ST + sub % TS;
-      if (tt >= M.ntiles || st >= M.ntiles || tt < st) continue;  // block-uniform
-      const Tile& T = Tt[sub / TS];
-      const Tile& S = St[sub % TS];
-      const bool mirror = tt > st;
-      const int ti0 = tt * kTile, sj0 = st * kTile;
-      const int nti = min(kTile, nc - ti0), nsj = min(kTile, nc - sj0);
-      // the near and vertex-sharing pairs of this tile pair (the relation is symmetric, so
-      // the same bits mark the transposed block)
-      const int moff = __ldg(M.tile_mask + static_cast<int64_t>(tt) * M.ntiles + st);
-      if (threadIdx.x < kTile)
-        skip[threadIdx.x] = moff >= 0 ? __ldg(M.masks + static_cast<int64_t>(moff) * kTile + threadIdx.x) : 0u;
-      __syncthreads();
-      const unsigned skip_it = it < nti ? skip[it] : ~0u;
-      const int k0 = kc * a.kchunk, k1 = min(a.nk, k0 + a.kchunk);
-      for (int kk = k0; kk < k1; ++kk) {
-        const double k = a.ks[kk];
-        float2* out = M.out + static_cast<long long>(kk) * nc * nc;
-        if (it < nti) {
-          for (int js = warp; js < nsj; js += kWarps) {
-            if ((skip_it >> js) & 1u) continue;
-            double ore[1][1], oim[1][1];
-            block_fp32<6, kHelmholtz, kSL, 1, 1, kPhaseRuntime>(T, it, S, js, rule, k, ore, oim);
-            const float2 v = make_float2(static_cast<float>(ore[0][0]), static_cast<float>(oim[0][0]));
-            out[static_cast<long long>(sj0 + js) * nc + ti0 + it] = v;
-            if (mirror) mir[js * (kTile + 1) + it] = v;
-          }
-        }
-        if (mirror) {
-          // the transposed block, entry (row sj0 + j, column ti0 + i), j fastest: coalesced
-          __syncthreads();
-          for (int idx = threadIdx.x; idx < kTile * kTile; idx += kThreads) {
-            const int i = idx / kTile, j = idx % kTile;
-            if (i < nti && j < nsj && !((skip[i] >> j) & 1u))
-              out[static_cast<long long>(ti0 + i) * nc + sj0 + j] = mir[j * (kTile + 1) + i];
-          }
-          __syncthreads();  // mir is reused by the next wavenumber
-        }
-      }
-      __syncthreads();  // the skip words are reused by the next tile pair
-    }
-  }
-}
-
-// Single-layer DP0 entry of one cell pair (test i, trial j) by the 6-point rule in FP64,
-// points and geometry from the grid arrays: phase referenced to the pair when
-// k (rad_i + rad_j) <= 0.8, else sincos_cw.
-__device__ double2 sl_dp0_pair_fp64(const CellSet& cs, int i, int j, const RegularRule& rule,
-                                    double k) {
-  const int64_t S = cs.stride;
-  const double dcx = g(cs.geom, kCx, cs.stride, i) - g(cs.geom, kCx, cs.stride, j);
-  const double dcy = g(cs.geom, kCy, cs.stride, i) - g(cs.geom, kCy, cs.stride, j);
-  const double dcz = g(cs.geom, kCz, cs.stride, i) - g(cs.geom, kCz, cs.stride, j);
-  const bool ref = k * (g(cs.geom, kRad, cs.stride, i) + g(cs.geom, kRad, cs.stride, j)) <=
-                   static_cast<double>(kSmallPhaseMax);
-  double kr0 = 0.0, pc = 1.0, ps = 0.0;
-  if (ref) {
-    const double r0sq = dcx * dcx + dcy * dcy + dcz * dcz;
-    kr0 = k * (r0sq * rsqrt_refined(r0sq));
-    sincos_cw(kr0, ps, pc);
-  }
-  double yq[6][3];
-#pragma unroll
-  for (int q = 0; q < 6; ++q)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) yq[q][d] = __ldg(cs.qpts + (q * 3 + d) * S + j);
-  double re = 0.0, im = 0.0;
-#pragma unroll 1
-  for (int p = 0; p < 6; ++p) {
-    const double x0 = __ldg(cs.qpts + (p * 3) * S + i), x1 = __ldg(cs.qpts + (p * 3 + 1) * S + i),
-                 x2 = __ldg(cs.qpts + (p * 3 + 2) * S + i);
-    double ur = 0.0, ui = 0.0;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const double dx = x0 - yq[q][0], dy = x1 - yq[q][1], dz = x2 - yq[q][2];
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      const double rinv = rsqrt_refined(r2);
-      const double r = r2 * rinv;
-      double sn, cs_;
-      if (ref)
-        sincos_small(fma(k, r, -kr0), sn, cs_);
-      else
-        sincos_cw(k * r, sn, cs_);
-      const double f = rule.w[q] * rinv;
-      ur = fma(f, cs_, ur);
-      ui = fma(f, sn, ui);
-    }
-    re = fma(rule.w[p], ur, re);
-    im = fma(rule.w[p], ui, im);
-  }
-  const double sc = g(cs.geom, kJdet, cs.stride, i) * g(cs.geom, kJdet, cs.stride, j) * kInv4Pi;
-  return make_double2((re * pc - im * ps) * sc, (re * ps + im * pc) * sc);
-}
-
-// The near pairs (no shared vertex) of every mesh and wavenumber: one thread per (pair,
-// wavenumber), wavenumber fastest.
-__global__ void __launch_bounds__(kThreads)
-    sweep_near_fp64(SweepArgs a, RegularRule rule) {
-  const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= a.near_begin[a.nmesh]) return;
-  int m = 0;
-  while (m + 1 < a.nmesh && t >= a.near_begin[m + 1]) ++m;
-  const SweepMesh& M = a.mesh[m];
-  const long long local = t - a.near_begin[m];
-  const int e = static_cast<int>(local / a.nk), kk = static_cast<int>(local % a.nk);
-  const int2 pr = __ldg(M.near_pairs + e);
-  const double2 v = sl_dp0_pair_fp64(M.cells, pr.x, pr.y, rule, a.ks[kk]);
-  const int nc = M.cells.ncells;
-  M.out[static_cast<long long>(kk) * nc * nc + static_cast<long long>(pr.y) * nc + pr.x] =
-      make_float2(static_cast<float>(v.x), static_cast<float>(v.y));
-}
-
-// The vertex-sharing pairs of every mesh and wavenumber by their Duffy rules: one warp
-// per (pair, wavenumber), wavenumber fastest; lanes over the rule's points.
-__global__ void __launch_bounds__(kThreads)
-    sweep_duffy_fp64(SweepArgs a, SingularRules rules) {
-  const long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= a.sing_begin[a.nmesh]) return;  // warp-uniform
-  int m = 0;
-  while (m + 1 < a.nmesh && w >= a.sing_begin[m + 1]) ++m;
-  const SweepMesh& M = a.mesh[m];
-  const long long local = w - a.sing_begin[m];
-  const int e = static_cast<int>(local / a.nk), kk = static_cast<int>(local % a.nk);
-  const double k = a.ks[kk];
-  const CellSet& cs = M.cells;
-  const int tc = __ldg(M.sing.test_cell + e), sc = __ldg(M.sing.trial_cell + e);
-  const int cfg = __ldg(M.sing.config + e);
-  double t0x[3], t1x[3], t0y[3], t1y[3], dv[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    t0x[d] = g(cs.geom, kT0x + d, cs.stride, tc);
-    t1x[d] = g(cs.geom, kT1x + d, cs.stride, tc);
-    t0y[d] = g(cs.geom, kT0x + d, cs.stride, sc);
-    t1y[d] = g(cs.geom, kT1x + d, cs.stride, sc);
-    dv[d] = g(cs.geom, kV0x + d, cs.stride, tc) - g(cs.geom, kV0x + d, cs.stride, sc);
-  }
-  const int off = __ldg(rules.offset + cfg), npts = __ldg(rules.offset + cfg + 1) - off;
-  // |k r| <= k (diam_x + diam_y): no reduction of the phase when that is below pi/4
-  const bool small_phase =
-      k * (g(cs.geom, kDiam, cs.stride, tc) + g(cs.geom, kDiam, cs.stride, sc)) <= 0.78;
-  const double2* txi = reinterpret_cast<const double2*>(rules.test_xi);
-  const double2* sxi = reinterpret_cast<const double2*>(rules.trial_xi);
-  double sr = 0.0, si = 0.0;
-  for (int ii = lane; ii < npts; ii += 32) {
-    const int i = off + ii;
-    const double2 xi = __ldg(txi + i), et = __ldg(sxi + i);
-    const double wt = __ldg(rules.w + i);
-    double r2 = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double dd = fma(xi.x, t0x[d], fma(xi.y, t1x[d], fma(-et.x, t0y[d], fma(-et.y, t1y[d], dv[d]))));
-      r2 = fma(dd, dd, r2);
-    }
-    const double rinv = rsqrt_refined(r2);
-    double sn, cs_;
-    if (small_phase)
-      sincos_taylor(k * r2 * rinv, sn, cs_);
-    else
-      sincos_cw(k * r2 * rinv, sn, cs_);
-    sr = fma(wt * rinv, cs_, sr);
-    si = fma(wt * rinv, sn, si);
-  }
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    sr += __shfl_xor_sync(0xffffffffu, sr, s);
-    si += __shfl_xor_sync(0xffffffffu, si, s);
-  }
-  if (lane == 0) {
-    const double scl = g(cs.geom, kJdet, cs.stride, tc) * g(cs.geom, kJdet, cs.stride, sc) * kInv4Pi;
-    const int nc = cs.ncells;
-    M.out[static_cast<long long>(kk) * nc * nc + static_cast<long long>(sc) * nc + tc] =
-        make_float2(static_cast<float>(sr * scl), static_cast<float>(si * scl));
-  }
-}
-
 size_t smem_bytes(int q, bool rel, bool queue, bool direct, bool cplx, int max_t, int max_s,
                   int nbt, int nbs, int acc_copies, bool mirror, bool pts, bool split_stage) {
   size_t b = 16;  // the mbarrier
@@ -1689,69 +1428,6 @@ cudaError_t take_stage_timeouts(unsigned* count) {
   if (e != cudaSuccess || *count == 0) return e;
   const unsigned zero = 0;
   return cudaMemcpyToSymbol(g_stage_timeouts, &zero, sizeof(unsigned));
-}
-
-size_t sweep_smem_bytes(int ts) {
-  size_t b = 16;  // the mbarrier
-  for (int t = 0; t < 2 * ts; ++t) {  // tiles without FP64 points
-    b += sizeof(double) * tile_doubles(6, false) + sizeof(float) * tile_floats(6, true) +
-         sizeof(int) * tile_ints(1);
-    b = (b + 15) & ~size_t(15);
-  }
-  return b + 2 * sizeof(long long) + sizeof(float2) * kTile * (kTile + 1) +
-         sizeof(unsigned) * kTile + 32;
-}
-
-namespace {
-template <int TS, int MINB>
-cudaError_t launch_sweep_shape(const SweepArgs& args, const RegularRule& rule, int blocks,
-                               cudaStream_t stream) {
-  const size_t smem = sweep_smem_bytes(TS);
-  auto fn = sweep_sl_dp0<TS, MINB>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e != cudaSuccess) {
-    cudaGetLastError();  // not sticky: clear it, so that it is not reported by a later launch
-    return e;
-  }
-  fn<<<blocks, kThreads, smem, stream>>>(args, rule);
-  return cudaGetLastError();
-}
-}  // namespace
-
-cudaError_t launch_sweep_sl(const SweepArgs& args, const RegularRule& rule,
-                            const SingularRules& rules, int blocks_per_sm, int sms,
-                            cudaStream_t stream) {
-  (void)rules;
-  if (rule.npts != 6) return cudaErrorInvalidValue;
-  if (args.tile_shape != 1 && args.tile_shape != 2) return cudaErrorInvalidValue;
-  const int blocks = blocks_per_sm * sms;
-  // the register cap follows the CTAs per SM asked for (at most 6)
-  if (args.tile_shape == 1)
-    return blocks_per_sm > 4 ? launch_sweep_shape<1, 6>(args, rule, blocks, stream)
-                             : launch_sweep_shape<1, 4>(args, rule, blocks, stream);
-  return blocks_per_sm > 4 ? launch_sweep_shape<2, 6>(args, rule, blocks, stream)
-                           : launch_sweep_shape<2, 4>(args, rule, blocks, stream);
-}
-
-cudaError_t launch_sweep_near_singular(const SweepArgs& args, const RegularRule& rule,
-                                       const SingularRules& rules, cudaStream_t stream) {
-  if (rule.npts != 6) return cudaErrorInvalidValue;
-  const long long nn = args.near_begin[args.nmesh], ns = args.sing_begin[args.nmesh];
-  if (nn > 0) {
-    const long long blocks = (nn + kThreads - 1) / kThreads;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    sweep_near_fp64<<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(args, rule);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  if (ns > 0) {
-    const long long blocks = (ns * 32 + kThreads - 1) / kThreads;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    sweep_duffy_fp64<<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(args, rules);
-    return cudaGetLastError();
-  }
-  return cudaSuccess;
 }
 
 cudaError_t launch_regular_dp0(const CellSet& test, const CellSet& trial,

@@ -263,6 +263,27 @@ __device__ __forceinline__ void reduced_cos_sin(float t, float& c, float& s) {
   s = (q == 0) ? sr : (q == 1) ? cr : (q == 2) ? -sr : -cr;
 }
 
+// reduced_cos_sin on two arguments, |t| up to 6e6: the multiple of pi/2 from the low bits of
+// t (2/pi) + 1.5 2^23, reduction and polynomials in packed instructions.
+__device__ __forceinline__ void reduced_cos_sin2(float2 t, float2& c, float2& s) {
+  const float2 big = ffma2(t, f2(0.636619772f), f2(12582912.f));
+  const float2 n = fadd2(big, f2(-12582912.f));
+  const float2 r = ffma2(n, f2(4.37113883e-8f), ffma2(n, f2(-1.57079637f), t));
+  const float2 z = fmul2(r, r);
+  const float2 cr = ffma2(z, ffma2(z, ffma2(z, ffma2(z, f2(2.437514408e-5f), f2(-1.388660219e-3f)),
+                                            f2(4.166661828e-2f)), f2(-4.999999968e-1f)), f2(1.0f));
+  const float2 sr = fmul2(r, ffma2(z, ffma2(z, ffma2(z, f2(-1.948277516e-4f), f2(8.331875683e-3f)),
+                                            f2(-1.666664881e-1f)), f2(1.0f)));
+  auto place = [](float x, float cx, float sx, float& co, float& so) {
+    const int q = __float_as_int(x);
+    const float cc = q & 1 ? sx : cx, ss = q & 1 ? cx : sx;
+    co = __int_as_float(__float_as_int(cc) ^ (((q + 1) & 2) << 30));
+    so = __int_as_float(__float_as_int(ss) ^ ((q & 2) << 30));
+  };
+  place(big.x, cr.x, sr.x, c.x, s.x);
+  place(big.y, cr.y, sr.y, c.y, s.y);
+}
+
 // e^{i theta} for an FP64 angle: the reduction by pi/2 in FP64 (two-part constant), the
 // series and the quadrant in FP32; absolute error ~1e-7.
 __device__ __forceinline__ void phase_cos_sin(double theta, float& c, float& s) {
