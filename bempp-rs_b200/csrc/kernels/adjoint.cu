@@ -19,10 +19,12 @@
 //
 // Regular pairs use 32 x 32 cell tiles (lane = test cell, both tiles staged in shared memory
 // by TMA bulk copies on an mbarrier with the regular kernels' bounded wait and timeout
-// counter); adjacent pairs use one warp per pair over their Duffy rule.  FP64 with the
+// counter); adjacent pairs use eight threads per pair over their Duffy rule.  FP64 with the
 // 6-point rule: adjoint_sl_orbits.  Other rules in FP64: adjoint_sl_regular.  Mixed:
 // far pairs (centroid distance >= 2 diameters) in FP32 with centroid-relative points and
 // the reference phase e^{ik r0} folded into the pair weight, as in regular.cu.
+#include <type_traits>
+
 #include "regular_fp64.cuh"
 
 namespace bempp_b200 {
@@ -657,98 +659,129 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
-struct CellGeo {
-  double v0[3], t0[3], t1[3], n[3], jdet;
-};
-
-__device__ __forceinline__ void load_geo(const CellSet& cs, int c, CellGeo& g) {
-  const int N = cs.stride;
-  for (int d = 0; d < 3; ++d) {
-    g.v0[d] = bempp_b200::g(cs.geom, kV0x + d, N, c);
-    g.t0[d] = bempp_b200::g(cs.geom, kT0x + d, N, c);
-    g.t1[d] = bempp_b200::g(cs.geom, kT1x + d, N, c);
-    g.n[d] = bempp_b200::g(cs.geom, kNx + d, N, c);
-  }
-  g.jdet = bempp_b200::g(cs.geom, kJdet, N, c);
-}
-
-// One warp per adjacent pair over its Duffy rule.
+// Adjacent pairs over their Duffy rules, kPairLanes threads per pair (pairs are grouped by
+// configuration, so a warp's pairs read the same points).  phi and psi are affine in the
+// points' coordinates, so the 18 vertex sums are combinations of five vector sums of
+// h (x - y), h = Re(c e^{ikr} (ikr - 1)) w / r^3, with factors 1, xi_0, xi_1, eta_0, eta_1: 17 sums per
+// pair to reduce over eight lanes, where a warp per pair reduced 22 over 32.
+// 66,500 pairs (5,120 triangles, order 4), k = 5, B200: 0.77 -> 0.47 ms.
+constexpr int kPairLanes = 8;
 __global__ void __launch_bounds__(256)
     adjoint_sl_singular(CellSet cs, SingularRules rules, SingularPairs pairs, double k,
                         const double2* __restrict__ lam, const double2* __restrict__ mu,
                         double* __restrict__ grad_cell, double* __restrict__ totals) {
-  const int lane = threadIdx.x & 31;
-  const int pair = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (pair >= pairs.npairs) return;
-  const int tc = pairs.test_cell[pair], sc = pairs.trial_cell[pair], cfg = pairs.config[pair];
-  CellGeo x, y;
-  load_geo(cs, tc, x);
-  load_geo(cs, sc, y);
+  const int64_t index = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) / kPairLanes;
+  const int sub = threadIdx.x % kPairLanes;
+  const bool valid = index < pairs.npairs;
+  const int pair = valid ? static_cast<int>(index) : 0;
+  const int tc = __ldg(pairs.test_cell + pair), sc = __ldg(pairs.trial_cell + pair),
+            cfg = __ldg(pairs.config + pair);
+  double tx[2][3], ty[2][3], dv[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    tx[0][d] = g(cs.geom, kT0x + d, cs.stride, tc);
+    tx[1][d] = g(cs.geom, kT1x + d, cs.stride, tc);
+    ty[0][d] = g(cs.geom, kT0x + d, cs.stride, sc);
+    ty[1][d] = g(cs.geom, kT1x + d, cs.stride, sc);
+    dv[d] = g(cs.geom, kV0x + d, cs.stride, tc) - g(cs.geom, kV0x + d, cs.stride, sc);
+  }
   const double2 li = lam[tc], mj = mu[sc];
   const double c_re = li.x * mj.x + li.y * mj.y, c_im = li.x * mj.y - li.y * mj.x;
-  const int off = rules.offset[cfg], npts = rules.offset[cfg + 1] - off;
+  const int off = __ldg(rules.offset + cfg), npts = valid ? __ldg(rules.offset + cfg + 1) - off : 0;
   // |k r| <= k (diam_x + diam_y) for a pair sharing a vertex: no phase reduction needed
   // when that is below pi/4
-  const bool small_phase = k * (bempp_b200::g(cs.geom, kDiam, cs.stride, tc) +
-                                bempp_b200::g(cs.geom, kDiam, cs.stride, sc)) <= 0.78;
-  double S0_re = 0.0, S0_im = 0.0, Sk_re = 0.0, Sk_im = 0.0;
-  double gx[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, gy[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-  for (int ii = lane; ii < npts; ii += 32) {
-    const int i = off + ii;
-    const double xi0 = rules.test_xi[2 * i], xi1 = rules.test_xi[2 * i + 1];
-    const double et0 = rules.trial_xi[2 * i], et1 = rules.trial_xi[2 * i + 1];
-    const double w = rules.w[i];
-    double d[3];
-    for (int c = 0; c < 3; ++c)
-      d[c] = (x.v0[c] + xi0 * x.t0[c] + xi1 * x.t1[c]) - (y.v0[c] + et0 * y.t0[c] + et1 * y.t1[c]);
-    const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    const double rinv = rsqrt_refined(r2);
-    const double r = r2 * rinv, kr = k * r;
-    double sn, csn;
-    if (small_phase)
-      sincos_taylor(kr, sn, csn);
-    else
-      sincos_cw(kr, sn, csn);
-    S0_re = fma(w * rinv, csn, S0_re);
-    S0_im = fma(w * rinv, sn, S0_im);
-    Sk_re = fma(w, csn, Sk_re);
-    Sk_im = fma(w, sn, Sk_im);
-    const double f_re = -csn - kr * sn, f_im = kr * csn - sn;
-    const double gs = w * (c_re * f_re - c_im * f_im) * rinv * rinv * rinv;
-    const double phi[3] = {1.0 - xi0 - xi1, xi0, xi1};
-    const double psi[3] = {1.0 - et0 - et1, et0, et1};
-    for (int a = 0; a < 3; ++a)
-      for (int c = 0; c < 3; ++c) {
-        gx[a][c] = fma(gs * phi[a], d[c], gx[a][c]);
-        gy[a][c] = fma(-gs * psi[a], d[c], gy[a][c]);
-      }
-  }
-  for (int s = 16; s > 0; s >>= 1) {
-    S0_re += __shfl_xor_sync(0xffffffffu, S0_re, s);
-    S0_im += __shfl_xor_sync(0xffffffffu, S0_im, s);
-    Sk_re += __shfl_xor_sync(0xffffffffu, Sk_re, s);
-    Sk_im += __shfl_xor_sync(0xffffffffu, Sk_im, s);
-    for (int a = 0; a < 3; ++a)
-      for (int c = 0; c < 3; ++c) {
-        gx[a][c] += __shfl_xor_sync(0xffffffffu, gx[a][c], s);
-        gy[a][c] += __shfl_xor_sync(0xffffffffu, gy[a][c], s);
-      }
-  }
-  if (lane != 0) return;
-  const double jj = x.jdet * y.jdet * kInv4Pi;
-  const double R0 = c_re * S0_re - c_im * S0_im;
-  double djx[3][3], djy[3][3];
-  jdet_gradient(x.t0, x.t1, x.n, djx);
-  jdet_gradient(y.t0, y.t1, y.n, djy);
-  for (int a = 0; a < 3; ++a)
-    for (int c = 0; c < 3; ++c) {
-      atomicAdd(grad_cell + static_cast<int64_t>(tc) * 9 + a * 3 + c,
-                jj * gx[a][c] + R0 * y.jdet * kInv4Pi * djx[a][c]);
-      atomicAdd(grad_cell + static_cast<int64_t>(sc) * 9 + a * 3 + c,
-                jj * gy[a][c] + R0 * x.jdet * kInv4Pi * djy[a][c]);
+  const bool small_phase =
+      fabs(k) * (g(cs.geom, kDiam, cs.stride, tc) + g(cs.geom, kDiam, cs.stride, sc)) <= 0.78;
+  const double2* txi = reinterpret_cast<const double2*>(rules.test_xi);
+  const double2* sxi = reinterpret_cast<const double2*>(rules.trial_xi);
+  double R0 = 0.0, dk = 0.0, v[5][3];
+#pragma unroll
+  for (int e = 0; e < 5; ++e)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[e][d] = 0.0;
+  auto points = [&](auto small) {
+#pragma unroll 1
+    for (int i = off + sub; i < off + npts; i += kPairLanes) {
+      const double2 xi = __ldg(txi + i), et = __ldg(sxi + i);
+      const double w = __ldg(rules.w + i);
+      double d[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        d[c] = fma(xi.x, tx[0][c], fma(xi.y, tx[1][c], fma(-et.x, ty[0][c], fma(-et.y, ty[1][c], dv[c]))));
+      const double r2 = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
+      const double rinv = rsqrt_refined(r2), kr = k * (r2 * rinv);
+      double sn, csn;
+      if constexpr (decltype(small)::value)
+        sincos_taylor(kr, sn, csn);
+      else
+        sincos_any(kr, sn, csn);
+      // Re(c e^{ikr}), Re(i c e^{ikr})
+      const double a = fma(c_re, csn, -c_im * sn), b = -fma(c_re, sn, c_im * csn);
+      const double wr = w * rinv;
+      R0 = fma(wr, a, R0);
+      dk = fma(w, b, dk);
+      const double h = wr * (rinv * rinv) * fma(kr, b, -a);
+      const double f[5] = {h, h * xi.x, h * xi.y, h * et.x, h * et.y};
+#pragma unroll
+      for (int e = 0; e < 5; ++e)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[e][c] = fma(f[e], d[c], v[e][c]);
     }
-  atomicAdd(totals, R0 * jj);
-  atomicAdd(totals + 1, (c_re * (-Sk_im) - c_im * Sk_re) * jj);
+  };
+  if (small_phase)
+    points(std::true_type{});
+  else
+    points(std::false_type{});
+#pragma unroll
+  for (int s = kPairLanes / 2; s > 0; s >>= 1) {
+    R0 += __shfl_xor_sync(0xffffffffu, R0, s);
+    dk += __shfl_xor_sync(0xffffffffu, dk, s);
+#pragma unroll
+    for (int e = 0; e < 5; ++e)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[e][c] += __shfl_xor_sync(0xffffffffu, v[e][c], s);
+  }
+  const double jx = g(cs.geom, kJdet, cs.stride, tc), jy = g(cs.geom, kJdet, cs.stride, sc);
+  const double jj = jx * jy * kInv4Pi;
+  // J and dJ/dk: one addition per CTA (one per pair queued at the two addresses)
+  double J = sub == 0 && valid ? R0 * jj : 0.0, K = sub == 0 && valid ? dk * jj : 0.0;
+#pragma unroll
+  for (int s = kPairLanes; s < 32; s <<= 1) {
+    J += __shfl_xor_sync(0xffffffffu, J, s);
+    K += __shfl_xor_sync(0xffffffffu, K, s);
+  }
+  __shared__ double part[2][8];
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = J;
+    part[1][threadIdx.x >> 5] = K;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sum += part[threadIdx.x][w];
+    atomicAdd(totals + threadIdx.x, sum);
+  }
+  // one thread per side of the pair
+  if (sub > 1 || !valid) return;
+  const int cell = sub == 0 ? tc : sc;
+  double t0[3], t1[3], n[3], dj[3][3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    t0[d] = sub == 0 ? tx[0][d] : ty[0][d];
+    t1[d] = sub == 0 ? tx[1][d] : ty[1][d];
+    n[d] = g(cs.geom, kNx + d, cs.stride, cell);
+  }
+  jdet_gradient(t0, t1, n, dj);
+  const double rj = R0 * (sub == 0 ? jy : jx) * kInv4Pi, sj = sub == 0 ? jj : -jj;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double p1 = sub == 0 ? v[1][c] : v[3][c], p2 = sub == 0 ? v[2][c] : v[4][c];
+    const double p[3] = {(v[0][c] - p1) - p2, p1, p2};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      atomicAdd(grad_cell + static_cast<int64_t>(cell) * 9 + a * 3 + c, fma(sj, p[a], rj * dj[a][c]));
+  }
 }
 
 // Per-cell-vertex gradients -> per-point gradients (npoints x 3).
@@ -807,8 +840,9 @@ cudaError_t launch_adjoint_sl(const CellSet& cs, const RegularRule& rule,
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (pairs.npairs > 0) {
-    adjoint_sl_singular<<<(pairs.npairs + 7) / 8, 256, 0, stream>>>(cs, rules, pairs, k, l2, m2,
-                                                                   grad_cell, totals);
+    const int per = 256 / kPairLanes;
+    adjoint_sl_singular<<<(pairs.npairs + per - 1) / per, 256, 0, stream>>>(cs, rules, pairs, k, l2,
+                                                                           m2, grad_cell, totals);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   cell_to_point_gradient<<<(cs.ncells + 255) / 256, 256, 0, stream>>>(cs, grad_cell, grad_points);
