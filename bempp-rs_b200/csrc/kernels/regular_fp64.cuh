@@ -39,8 +39,8 @@
 //   (both orders of a pair at once) 17.7 -> 13.2, hypersingular P1 9.5 -> 7.3; Helmholtz
 //   k = 8 single layer DP0 15.8 -> 14.8, double layer P1 39.8 -> 36.9, hypersingular P1
 //   28.0 -> 21.7; 5,120 triangles, k = 8 (phases beyond 0.8): single layer 1.61 -> 1.18;
-//   2,048 triangles, 37-point rule: double layer P1 10.7 -> 4.2 (both orders at once);
-//   80 triangles, 37-point rule: single layer DP0 0.374 -> 0.022.
+//   2,048 triangles, 37-point rule: double layer P1 10.7 -> 4.0 (both orders at once);
+//   80 triangles, 37-point rule: single layer DP0 0.374 -> 0.021.
 // In FP64 issue slots the double layer needs about 19 per point pair for both orders (26
 // before), the hypersingular operator 11 (15), the Helmholtz single layer 29 (33).
 #pragma once
@@ -220,6 +220,13 @@ struct Traits {
   // test points of a point_block: enough chains to fill the pipe within the registers
   static constexpr int kPoints =
       KER == kHelmholtz && (PAIRED || (NBS == 3 && OP != kSL)) ? 2 : 4;
+  // trial points per turn of its loop: two where the registers hold both (37-point rule, 2,048
+  // triangles, one -> two: Laplace single layer DP0 2.35 -> 2.23 ms, double layer P1 4.26 -> 4.03,
+  // hypersingular 2.40 -> 2.24; Helmholtz single layer DP0 8.98 -> 8.43), one where they spill or
+  // cost a CTA (16-point rule, two bodies of 1,500 and 1,200: double layer P1 0.60 -> 0.67;
+  // Helmholtz single layer P1 1.77 -> 2.26, hypersingular 2.22 -> 2.36)
+  static constexpr int kTrialUnroll =
+      KER == kLaplace ? (OP == kDL && !PAIRED && NBT * NBS == 9 ? 1 : 2) : (NBT * NBS == 1 ? 2 : 1);
 };
 
 // Scalars of one cell pair (test cell = the lane's, trial cell js).
@@ -482,7 +489,7 @@ __device__ __forceinline__ void point_block(const PairGeometry& p, double ex0, d
         if constexpr (PAIRED) V[part][i][b] = 0.0;
       }
     }
-#pragma unroll 1
+#pragma unroll(Tr::kTrialUnroll)
   for (int q = 0; q < Q; ++q) {
     const double2* e = reinterpret_cast<const double2*>(rt + kRuleStride * q);
     const double2 ab = e[0], wp = e[1], pp = NBS == 3 ? e[2] : make_double2(0.0, 0.0);
