@@ -499,6 +499,7 @@ void assemble_device(BoundaryAssemblerT& a, SpaceT& trial, SpaceT& test, void* d
                              (test.grid->max_circumradius() + trial.grid->max_circumradius()) *
                              (1.0 + 1e-6);
   ra.small_phase = phase_bound <= 0.8 ? 1 : 0;
+  ra.phase_bound = phase_bound;
   // one P1 / DP1 space, double layer or its adjoint (mixed precision: the 6-point rule and,
   // for Helmholtz, phases referenced to the pair): the pair (i, j) and the pair (j, i) share
   // their kernel values, so both blocks of a tile pair come from one pass (one-launch

@@ -192,27 +192,33 @@ __device__ __forceinline__ void sincos_cw(double t, double& s, double& c) {
   s = (q == 0) ? sr : (q == 1) ? cr : (q == 2) ? -sr : -cr;
 }
 
-// sincos_small of N arguments, step by step.
-template <int N>
+// sincos_small of N arguments, step by step; SHORT: |t| <= 0.42.
+template <int N, bool SHORT = false>
 __device__ __forceinline__ void sincos_small_n(const double t[N], double s[N], double c[N]) {
-  constexpr double P[6] = {2.0657616391477202e-09,  -2.755574396426964e-07, 2.4801582078024058e-05,
+  constexpr int kTerms = SHORT ? 5 : 6;
+  // |t| <= 0.42: interpolation of the two series at Chebyshev points, errors 1.2e-16, 4e-18
+  constexpr double P5[5] = {-2.746539758703359e-07, 2.4801445491762405e-05, -0.0013888888799568808,
+                            0.04166666666646974, -0.4999999999999993};
+  constexpr double Q5[5] = {-2.4981384587602678e-08, 2.7557210109293225e-06, -0.00019841269772540994,
+                            0.00833333333331818, -0.1666666666666666};
+  constexpr double P6[6] = {2.0657616391477202e-09,  -2.755574396426964e-07, 2.4801582078024058e-05,
                            -0.0013888888881056654, 0.04166666666662371,    -0.4999999999999996};
-  constexpr double Q[6] = {1.5912864224903485e-10, -2.5051057394492127e-08, 2.7557315738586845e-06,
+  constexpr double Q6[6] = {1.5912864224903485e-10, -2.5051057394492127e-08, 2.7557315738586845e-06,
                            -0.00019841269836043575, 0.008333333333330467,   -0.16666666666666663};
   double z[N], p[N], q[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) z[i] = t[i] * t[i];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    p[i] = P[0];
-    q[i] = Q[0];
+    p[i] = SHORT ? P5[0] : P6[0];
+    q[i] = SHORT ? Q5[0] : Q6[0];
   }
 #pragma unroll
-  for (int j = 1; j < 6; ++j) {
+  for (int j = 1; j < kTerms; ++j) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) p[i] = fma(p[i], z[i], P[j]);
+    for (int i = 0; i < N; ++i) p[i] = fma(p[i], z[i], SHORT ? P5[j % 5] : P6[j]);
 #pragma unroll
-    for (int i = 0; i < N; ++i) q[i] = fma(q[i], z[i], Q[j]);
+    for (int i = 0; i < N; ++i) q[i] = fma(q[i], z[i], SHORT ? Q5[j % 5] : Q6[j]);
   }
 #pragma unroll
   for (int i = 0; i < N; ++i) c[i] = fma(z[i], p[i], 1.0);

@@ -60,6 +60,7 @@ struct RegularArgs {
   void* out;         // column-major output
   int small_phase = 0;   // Helmholtz, mixed: k (max rad_test + max rad_trial) <= 0.8, so
                          // |k (r - r0)| <= 0.8 for every far pair (no phase reduction)
+  double phase_bound = 1e300;  // k (max rad_test + max rad_trial)
   NearArgs near{};       // mixed: near field (null: near pairs found per pair in the kernel)
   int symmetric = 0;     // 1: test and trial are one space and the operator is symmetric
                          // (SL, HS): only tile pairs (tx >= sy) are computed, then mirrored;

@@ -37,12 +37,12 @@
 // Regular part on a B200, coordinate differences in 32 x 32 tiles per CTA -> this form:
 //   20,480 triangles, 6-point rule: Laplace single layer DP0 6.55 -> 5.05 ms, double layer P1
 //   (both orders of a pair at once) 17.7 -> 13.2, hypersingular P1 9.5 -> 7.3; Helmholtz
-//   k = 8 single layer DP0 15.8 -> 14.8, double layer P1 39.8 -> 36.9, hypersingular P1
-//   28.0 -> 21.7; 5,120 triangles, k = 8 (phases beyond 0.8): single layer 1.61 -> 1.18;
+//   k = 8 single layer DP0 15.8 -> 12.6, double layer P1 39.8 -> 35.7, hypersingular P1
+//   28.0 -> 21.1; 5,120 triangles, k = 8 (phases beyond 0.8): single layer 1.61 -> 1.18;
 //   2,048 triangles, 37-point rule: double layer P1 10.7 -> 4.0 (both orders at once);
 //   80 triangles, 37-point rule: single layer DP0 0.374 -> 0.021.
 // In FP64 issue slots the double layer needs about 19 per point pair for both orders (26
-// before), the hypersingular operator 11 (15), the Helmholtz single layer 29 (33).
+// before), the hypersingular operator 11 (15), the Helmholtz single layer 27 to 29 (33).
 #pragma once
 
 #include <algorithm>
@@ -59,8 +59,10 @@ constexpr int kChunk = 16;   // most trial cells per CTA
 constexpr int kBand = 16;    // trial tiles per band of a tx >= sy launch (see tile_order.h)
 
 // Phases of Helmholtz kernels: referenced to the pair, |k (r - r0)| <= 0.8 for every pair
-// of the launch (checked on the host), or any phase k r reduced by multiples of pi/2.
-enum Phase : int { kReferenced = 0, kAnyPhase = 1 };
+// of the launch (checked on the host), or any phase k r reduced by multiples of pi/2; kShort:
+// referenced and at most 0.42, two terms less (20,480 triangles, k = 8, 0.41 at most, B200:
+// whole single layer DP0 13.5 -> 12.7 ms).
+enum Phase : int { kReferenced = 0, kAnyPhase = 1, kShort = 2 };
 
 // Rows of a staged tile (every row of the grid's geometry) after geometry_to_offsets: vertex
 // 0 becomes what the rounded centroid lacks, the tangents become g_0, g_1 and the last
@@ -174,14 +176,14 @@ __device__ __forceinline__ void kernel_values(const double r2[N], double k, doub
   double kr[N], sn[N], cs[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) kr[i] = r2[i] * rinv[i];  // r, times k below
-  if constexpr (PH == kReferenced) {
+  if constexpr (PH != kAnyPhase) {
     double t[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       if (kGrad) kr[i] *= k;
       t[i] = kGrad ? kr[i] - kr0 : fma(k, kr[i], -kr0);
     }
-    sincos_small_n<N>(t, sn, cs);
+    sincos_small_n<N, PH == kShort>(t, sn, cs);
   } else {
 #pragma unroll
     for (int i = 0; i < N; ++i) kr[i] *= k;
@@ -920,7 +922,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
     PairGeometry p;
     pair_geometry<KER, OP, NBT, NBS, PAIRED>(T, it, S, js, kScaledFactors ? sc : 1.0, p);
     double kr0 = 0.0;
-    if constexpr (kC && PH == kReferenced) kr0 = k * (p.r0 * rsqrt_refined(p.r0));
+    if constexpr (kC && PH != kAnyPhase) kr0 = k * (p.r0 * rsqrt_refined(p.r0));
     Blocks<NP, NBT, NBS, PAIRED> blk;
     if constexpr (ORBITS) {
       pair_orbits<KER, OP, NBT, NBS, PAIRED, PH>(p, T, it, S, js, rule, k, kr0, blk);
@@ -959,7 +961,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
         point_block<KER, OP, NBT, NBS, PAIRED, PH, 1>(p, ex0, hx, ex1, rt, Yq, Q, rest, k, kr0, blk);
     }
     // ---- the pair's block: reference phase, scale, curls
-    if constexpr (kC && PH == kReferenced) {
+    if constexpr (kC && PH != kAnyPhase) {
       double ps, pc;
       sincos_any(kr0, ps, pc);
       if constexpr (Tr::kHSSum) {
@@ -1270,6 +1272,13 @@ inline PointRule point_rule(const RegularRule& r) {
     for (int i = 0; i < kPointFields; ++i) p.p[q][i] = f[i];
   }
   return p;
+}
+
+// The largest offset of a point of such a rule from the centroid, in circumradii.
+inline double orbit_reach(const RegularRule& r) {
+  double g = 0.0;
+  for (int o = 0; o < 2; ++o) g = fmax(g, fabs((r.phi[0][3 * o] - 1.0 / 3.0) * 1.5));
+  return g;
 }
 
 // Two S21 orbits, points in vertex order (point b of an orbit has its largest or smallest
