@@ -1298,6 +1298,23 @@ inline bool has_orbit_form(const RegularRule& r) {
 
 constexpr int kSMs = 148;
 
+template <int KER, int NBS, bool DIRECT, bool PAIRED>
+inline void set_accumulator(Shape& sh, const SpaceTiles& tt, const SpaceTiles& st) {
+  // accumulators of up to 12 KB per warp: three CTAs per SM stay resident; larger ones
+  // (discontinuous P1, meshes whose tiles touch many DOFs) are replaced by direct adds
+  sh.cap = 0;
+  sh.gather = 0;
+  if (!DIRECT) {
+    const int chunk_dofs = std::min(st.max_tile_dofs, sh.ns * NBS);
+    // (a shorter chunk lies within one of kChunk cells)
+    sh.cap = tt.max_tile_dofs * std::min(chunk_dofs, st.max_chunk_dofs);
+    const size_t bytes = sizeof(double) * static_cast<size_t>(sh.cap) * (KER == kHelmholtz ? 2 : 1) *
+                         (PAIRED ? 2 : 1);
+    sh.gather = bytes <= (size_t(20) << 10) ? 1 : 0;
+    if (!sh.gather) sh.cap = 0;
+  }
+}
+
 template <bool ORBITS, int KER, int OP, int NBT, int NBS, bool DIRECT, bool PAIRED, int PH,
           bool SPLIT>
 cudaError_t launch_shape(const CellSet& test, const SpaceTiles& tt, const CellSet& trial,
@@ -1311,19 +1328,7 @@ cudaError_t launch_shape(const CellSet& test, const SpaceTiles& tt, const CellSe
   const long long blocks = units * (kTile / sh.ns);
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   if (blocks <= 0) return cudaSuccess;
-  // accumulators of up to 12 KB per warp: three CTAs per SM stay resident; larger ones
-  // (discontinuous P1, meshes whose tiles touch many DOFs) are replaced by direct adds
-  sh.cap = 0;
-  sh.gather = 0;
-  if (!DIRECT) {
-    const int chunk_dofs = std::min(st.max_tile_dofs, sh.ns * NBS);
-    const int known = sh.ns == kChunk ? std::min(chunk_dofs, st.max_chunk_dofs) : chunk_dofs;
-    sh.cap = tt.max_tile_dofs * known;
-    const size_t bytes = sizeof(double) * static_cast<size_t>(sh.cap) * (KER == kHelmholtz ? 2 : 1) *
-                         (PAIRED ? 2 : 1);
-    sh.gather = bytes <= (size_t(20) << 10) ? 1 : 0;
-    if (!sh.gather) sh.cap = 0;
-  }
+  set_accumulator<KER, NBS, DIRECT, PAIRED>(sh, tt, st);
   const Layout L = layout<ORBITS, KER, OP, NBT, NBS, DIRECT, PAIRED, SPLIT>(
       rule.npts, sh.ns, sh.gather, sh.cap, a.symmetric);
   auto fn = regular_fp64<ORBITS, KER, OP, NBT, NBS, DIRECT, PAIRED, PH, SPLIT>;
@@ -1347,6 +1352,38 @@ cudaError_t launch_shape(const CellSet& test, const SpaceTiles& tt, const CellSe
   return cudaGetLastError();
 }
 
+// Trial cells per CTA of the 6-point rule's kernels (`tiles`: CTAs that whole tiles would take).
+// A CTA costs its staging, incidence and flush (about `fixed` trial cells' time per wave of
+// the CTAs that an SM holds, and the adds of its block); a trial cell costs one unit per CTA
+// on the SM, but not less than four (one warp's latency).  The least estimate, longer chunks on
+// ties.  B200, shorter chunks until 888 CTAs -> this: 640 triangles, one space, Laplace double
+// layer P1 53 -> 35 us, single layer DP0 27 -> 19; 1,280: double layer 91 -> 77; two bodies of
+// 800 and 700, hypersingular 46 -> 41; Helmholtz, k = 10: 1,280 hypersingular 168 -> 142, two
+// bodies double layer 156 -> 123.
+template <int KER, int OP, int NBT, int NBS, bool DIRECT, bool PAIRED>
+inline int orbit_chunk(long long tiles, Shape sh, const SpaceTiles& tt, const SpaceTiles& st,
+                       int npts, int symmetric) {
+  constexpr bool kC = KER == kHelmholtz;
+  const long long fixed = (DIRECT ? 5 : 10) / (kC ? 2 : 1), adds = DIRECT ? 0 : kC ? 1 : 2;
+  int best = kChunk;
+  long long least = 0;
+  for (int ns = kChunk; ns >= 1; ns /= 2) {
+    sh.ns = ns;
+    set_accumulator<KER, NBS, DIRECT, PAIRED>(sh, tt, st);
+    const size_t smem = layout<true, KER, OP, NBT, NBS, DIRECT, PAIRED, false>(
+                            npts, ns, sh.gather, sh.cap, symmetric).total + 1024;
+    const long long resident = std::max<long long>(
+        1, std::min<long long>(min_ctas<true, KER, OP, NBT, NBS, PAIRED>(), (size_t(227) << 10) / smem));
+    const long long n = (tiles * (kTile / ns) + kSMs - 1) / kSMs;  // CTAs of the fullest SM
+    const long long cost = (n + resident - 1) / resident * fixed + n * adds + ns * std::max(4LL, n);
+    if (ns == kChunk || cost < least) {
+      least = cost;
+      best = ns;
+    }
+  }
+  return best;
+}
+
 template <bool ORBITS, int KER, int OP, int NBT, int NBS, bool DIRECT, bool PAIRED, int PH>
 cudaError_t launch_one(const CellSet& test, const SpaceTiles& tt, const CellSet& trial,
                        const SpaceTiles& st, const RegularRule& rule, const RegularArgs& a,
@@ -1361,11 +1398,13 @@ cudaError_t launch_one(const CellSet& test, const SpaceTiles& tt, const CellSet&
   sh.ntt = (test.ncells + kTile - 1) / kTile;
   sh.ty0 = a.trial_tile0;
   sh.ty1 = a.trial_tile0 + ny;
-  // CTAs of full chunks; shorter chunks until the chip has about three CTAs per SM twice over
   long long tiles = static_cast<long long>((sh.ntt + kWarps - 1) / kWarps) * ny;
   if (a.symmetric) tiles = (tiles + 1) / 2;
   sh.ns = kChunk;
-  while (sh.ns > 1 && tiles * (kTile / sh.ns) < 6 * kSMs) sh.ns /= 2;
+  if constexpr (ORBITS)
+    sh.ns = orbit_chunk<KER, OP, NBT, NBS, DIRECT, PAIRED>(tiles, sh, tt, st, rule.npts, a.symmetric);
+  else  // shorter chunks until the chip has about three CTAs per SM twice over
+    while (sh.ns > 1 && tiles * (kTile / sh.ns) < 6 * kSMs) sh.ns /= 2;
   if constexpr (!ORBITS) {
     // still too few warps: the rule's test points over the four warps of a CTA
     if (tiles * (kTile / sh.ns) < 2 * kSMs && rule.npts >= 12) {
