@@ -1,5 +1,5 @@
 // Batched Helmholtz single-layer DP0 frequency sweep: one persistent, CUDA-graph-captured
-// launch over many wavenumbers and meshes of uneven size (the regular.cu kernel
+// launch over many wavenumbers and meshes of uneven size (the sweep.cu kernel
 // sweep_sl_dp0), with a small autotuner.
 //
 // Plan.  Work items are (mesh, chunk of wavenumbers, tile pair test tile >= trial tile:
@@ -10,9 +10,8 @@
 // Autotuner.  The free parameters are the tile shape of a work item (1 x 1 or 2 x 2 pairs
 // of 32-cell tiles staged together: reuse of staged tiles versus shared memory per CTA),
 // the wavenumbers per work item (k-chunk: more reuse of a staged tile pair versus finer
-// load balance) and the CTAs per SM of the persistent grid (which also sets the register
-// cap of the kernel: 4 or fewer CTAs allow 128 registers, 5 or 6 allow 80).  Each
-// candidate runs the kernel on a leading slice of the work items (the first 1/16th, at
+// load balance; eight of them share a cell pair's moments) and the CTAs per SM of the
+// persistent grid.  Each candidate runs the kernel on a leading slice of the work items (the first 1/16th, at
 // least 148 x 8 items) timed with CUDA events; the fastest is kept per (device, mesh
 // sizes, number of wavenumbers) for the life of the process.  The quadrature order is not
 // a parameter: the 6-point rule is part of the problem (another order gives another

@@ -566,9 +566,9 @@ __device__ __forceinline__ void far_sums_x2(const Tile& T, int it, const Tile& S
 // space on both sides (the paired launch): the FP32 packed loop of far_sums_x2 with the
 // phase referenced to the pair (|k (r - r0)| <= 0.8, the launch's bound), one kernel value
 // per point pair for DL(test i, trial j) (the normal factor (x_p - y).n_j per test point)
-// and DL(test j, trial i) (the factor (y_q - x).n_i per point pair, folded per test point
-// like block_fp64_dl_pair); geometry, the reference phase e^{ik r0} and the blocks' final
-// scaling in FP64.  dij / dji as in block_fp64_dl_pair.
+// and DL(test j, trial i) (the factor (y_q - x).n_i per point pair, folded per test point);
+// geometry, the reference phase e^{ik r0} and the blocks' final scaling in FP64.  dij: the block
+// of (test i, trial j), dji: of (test j, trial i), transposed to the same indices.
 template <int QT, int KER>
 __device__ __forceinline__ void block_fp32_dl_pair(const Tile& T, int it, const Tile& S, int js,
                                                    const RegularRule& rule, double k,
