@@ -314,13 +314,6 @@ __device__ __forceinline__ void lagrange_basis(double x, double y, double v[NB],
     }
   }
 }
-
-// P1 basis on the reference triangle: phi0 = 1 - x - y, phi1 = x, phi2 = y.
-__device__ __forceinline__ void p1_basis(double x, double y, double* phi) {
-  phi[0] = 1.0 - x - y;
-  phi[1] = x;
-  phi[2] = y;
-}
 #endif  // __CUDACC__
 
 }  // namespace bempp_b200

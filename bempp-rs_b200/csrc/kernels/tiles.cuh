@@ -90,31 +90,6 @@ __device__ inline void load_ldof(const Tile& t, int c0, int n, const uint8_t* ce
   }
 }
 
-// Whole tile by plain loads from all threads (rows of the padded grid arrays; the
-// padding cells of the last tile come along and are never used).
-__device__ inline void load_tile(const Tile& t, const CellSet& cs, int c0, int n, int q, bool mixed,
-                          const uint8_t* cell_ldof, int nb) {
-  const int64_t S = cs.stride;
-  for (int idx = threadIdx.x; idx < 3 * q * kTile; idx += kThreads) {
-    const int c = idx % kTile, pd = idx / kTile;
-    t.pts[idx] = __ldg(cs.qpts + pd * S + c0 + c);
-  }
-  if (mixed)
-    for (int idx = threadIdx.x; idx < qrel_rows(q) * kTile; idx += kThreads) {
-      const int c = idx % kTile, r = idx / kTile;
-      t.rel[idx] = __ldg(cs.qrel + r * S + c0 + c);
-    }
-  for (int idx = threadIdx.x; idx < kTileFields * kTile; idx += kThreads) {
-    const int c = idx % kTile, f = idx / kTile;
-    t.geo[idx] = __ldg(cs.geom + (kT0x + f) * S + c0 + c);
-  }
-  for (int idx = threadIdx.x; idx < 3 * kTile; idx += kThreads) {
-    const int c = idx % kTile, v = idx / kTile;
-    t.vid[idx] = __ldg(cs.vids + v * S + c0 + c);
-  }
-  load_ldof(t, c0, n, cell_ldof, nb);
-}
-
 // One cell's FP64 quadrature points and geometry into column c of a tile (the staging of
 // a single lane).
 __device__ inline void stage_cell(const Tile& t, int c, const CellSet& cs, int cell, int q) {
