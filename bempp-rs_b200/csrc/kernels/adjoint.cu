@@ -573,9 +573,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int nti = min(kTile, cs.ncells - ti0), nsj = min(kTile, cs.ncells - sj0);
   extern __shared__ __align__(16) unsigned char smem[];
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);  // completion of the tile copies
-  constexpr size_t kTileBytes = kStagedBytes;
-  const Tile T = tile_at(smem + 16), S = tile_at(smem + 16 + kTileBytes);
-  double* jx = reinterpret_cast<double*>(smem + 16 + 2 * kTileBytes);  // d jdet / d V, [e * kTile + c]
+  const Tile T = tile_at(smem + 16), S = tile_at(smem + 16 + kTileStride);
+  double* jx = reinterpret_cast<double*>(smem + 16 + 2 * kTileStride);  // d jdet / d V, [e * kTile + c]
   double* jy = jx + 9 * kTile;
   double* s_test = jy + 9 * kTile;                   // [warp][9][kTile] test-cell gradients
   double* s_trial = s_test + kWarps * 9 * kTile;     // [kTile][9] trial-cell gradients
@@ -622,7 +621,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     jdet_gradient(t0, t1, n, dj);
 #pragma unroll
     for (int e = 0; e < 9; ++e) (warp == 0 ? jx : jy)[e * kTile + it] = dj[e / 3][e % 3];
-    geometry_to_offsets(t, it);
+    geometry_to_offsets(t, it, rule.reach);
   }
   __syncthreads();
 
@@ -824,7 +823,7 @@ cudaError_t launch_adjoint_sl(const CellSet& cs, const RegularRule& rule,
   const double2* l2 = reinterpret_cast<const double2*>(lam);
   const double2* m2 = reinterpret_cast<const double2*>(mu);
   if (!mixed && fp64::has_orbit_form(rule)) {
-    const size_t bytes = 16 + 2 * fp64::kStagedBytes +
+    const size_t bytes = 16 + 2 * fp64::kTileStride +
                          sizeof(double) * ((2 * 9 + (kWarps + 1) * 9) * kTile + 2);
     e = cudaFuncSetAttribute(adjoint_sl_orbits, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(bytes));

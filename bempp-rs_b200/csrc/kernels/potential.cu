@@ -39,6 +39,7 @@ constexpr int kGroup = 6;  // rule points per kernel evaluation (their chains hi
 
 struct PotentialRule {
   int npts;
+  double reach;                     // see fp64::rule_reach
   double ab[kMaxRegularPoints][2];  // coordinates along g_0, g_1
   double w[kMaxRegularPoints][6];   // weight times basis values
 };
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   double* ab = len + kTile * Q;               // [2 * q]
   double* wt = ab + 2 * Q;                    // [q * NB + b]
   int* dof = reinterpret_cast<int*>(wt + NB * Q);  // [cell * NB + b]
-  for (int i = threadIdx.x; i < fp64::kRows * kTile; i += kThreads)
+  for (int i = threadIdx.x; i < kNumGeomFields * kTile; i += kThreads)
     S.geo[i] = __ldg(trial.geom + static_cast<int64_t>(i / kTile) * trial.stride + c0 + i % kTile);
   for (int i = threadIdx.x; i < Q; i += kThreads) {
     ab[2 * i] = rule.ab[i][0];
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                                          : __ldg(st.cell_dofs + e);
   }
   __syncthreads();
-  if (threadIdx.x < kTile) fp64::geometry_to_offsets(S, threadIdx.x);
+  if (threadIdx.x < kTile) fp64::geometry_to_offsets(S, threadIdx.x, rule.reach);
   __syncthreads();
   for (int i = threadIdx.x; i < kTile * Q; i += kThreads) {
     const int c = i % kTile, q = i / kTile;
@@ -199,6 +200,7 @@ cudaError_t launch_nb(const double* points, int npoints, const CellSet& trial,
   constexpr int NP = KER == kHelmholtz ? 2 : 1;
   PotentialRule r{};
   r.npts = rule.npts;
+  r.reach = fp64::rule_reach(rule);
   for (int q = 0; q < rule.npts; ++q) {
     r.ab[q][0] = rule.phi[0][q] - rule.phi[2][q];
     r.ab[q][1] = rule.phi[1][q] - rule.phi[2][q];

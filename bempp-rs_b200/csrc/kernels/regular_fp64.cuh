@@ -16,9 +16,12 @@
 //   * any other rule: A_p + |y_q - c_y|^2 + alpha_q W0_p + beta_q W1_p, (alpha, beta) the
 //     coordinates of the point along g_0, g_1: three operations, the rule's constants
 //     loaded once for four test points (point_block).
-// The terms are offsets within a cell, so nothing cancels beyond what |x - y| itself does;
-// the centroids' rounding, which would shift every point of a cell alike, is kept beside
-// them and enters dc.
+// The centroids' rounding, which would shift every point of a cell alike, is kept beside
+// the offsets and enters dc.  The terms are as large as H^2, H = |dc| and both cells' extents
+// together, so the sum is off by eps H^2 and 1/r by eps (H/r)^2, where differences of
+// coordinates lose eps |x| / r.  Pairs whose rule points may be closer than H / 16 (nearly in
+// contact without a shared vertex; see close_pair) are therefore integrated from the
+// components of x - y (pair_by_components).
 // P1 basis functions on an S21 orbit take two values, so U_b = sum_q w_q phi_b(q) K_q is
 // c S + d K_b with S the orbit's sum: 12 operations per 6 points instead of 18.
 //
@@ -66,12 +69,16 @@ enum Phase : int { kReferenced = 0, kAnyPhase = 1, kShort = 2 };
 
 // Rows of a staged tile (every row of the grid's geometry) after geometry_to_offsets: vertex
 // 0 becomes what the rounded centroid lacks, the tangents become g_0, g_1 and the last
-// three rows |g_0|^2, |g_1|^2, |g_2|^2.
-enum Row : int { rL = kV0x, rG0 = kT0x, rG1 = kT1x, rN = kNx, rJ = kJdet, rC = kCx, rE = kDiam };
+// three rows |g_0|^2, |g_1|^2, |g_2|^2.  One more row: the cell's part of the distance of the
+// centroids within which close_pair looks at a pair.
+enum Row : int { rL = kV0x, rG0 = kT0x, rG1 = kT1x, rN = kNx, rJ = kJdet, rC = kCx, rE = kDiam,
+                 rR = kNumGeomFields };
 static_assert(kV0x == 0 && kRad == kDiam + 1 && kH == kDiam + 2, "three rows for the squared lengths");
-constexpr int kRows = kNumGeomFields;
+constexpr int kRows = kNumGeomFields + 1;
 
+// reach: every rule point of a cell lies in the triangle c + reach (g_0, g_1, g_2).
 struct OrbitRule {
+  double reach;
   double g[2], g2[2];  // gamma, gamma^2
   double w[2];         // weight of each point
   double c[2], d[2];   // w (1 - gamma) / 3, w gamma: w phi_b(q) = c + d [b = q]
@@ -83,6 +90,7 @@ struct OrbitRule {
 constexpr int kPointFields = 6;
 struct PointRule {
   int npts;
+  double reach;
   double p[kMaxRegularPoints][kPointFields];
 };
 
@@ -212,6 +220,21 @@ struct Blocks {
   double s[NP];
 };
 
+template <int NP, int NBT, int NBS, bool PAIRED>
+__device__ __forceinline__ void clear(Blocks<NP, NBT, NBS, PAIRED>& blk) {
+#pragma unroll
+  for (int part = 0; part < NP; ++part) {
+    blk.s[part] = 0.0;
+#pragma unroll
+    for (int a = 0; a < NBT; ++a)
+#pragma unroll
+      for (int b = 0; b < NBS; ++b) {
+        blk.f[part][a][b] = 0.0;
+        if constexpr (PAIRED) blk.t[part][a][b] = 0.0;
+      }
+  }
+}
+
 template <int KER, int OP, int NBT, int NBS, bool PAIRED>
 struct Traits {
   static constexpr int kParts = KER == kHelmholtz ? 2 : 1;
@@ -219,6 +242,9 @@ struct Traits {
   static constexpr bool kBlock = OP != kHS || KER == kHelmholtz;   // f is needed
   static constexpr bool kTestFactor = OP == kDL || PAIRED;         // (x_p - y).n_y
   static constexpr bool kTrialFactor = OP == kADL || PAIRED;       // (y_q - x).n_x
+  // the normal factors carry jdet_x jdet_y / (4 pi) where no phase is left to multiply with
+  template <int PH>
+  static constexpr bool kScaledFactors = (kTestFactor || kTrialFactor) && (KER == kLaplace || PH == kAnyPhase);
   // test points of a point_block: enough chains to fill the pipe within the registers
   static constexpr int kPoints =
       KER == kHelmholtz && (PAIRED || (NBS == 3 && OP != kSL)) ? 2 : 4;
@@ -277,6 +303,62 @@ __device__ __forceinline__ void pair_geometry(const Tile& T, int it, const Tile&
   }
 }
 
+// Whether rule points of a pair may be closer than kSeparation times `limit`, the sum of the
+// cells' rR rows.  Not where |dc| reaches the limit; nearer pairs are looked at along dc, where
+// the points of a cell lie within reach times its vertices.  An ordinary mesh has no such
+// pair with the 6-point rule; with 37 points and anisotropic cells about one cell in ten has one.
+constexpr double kSeparation = 0.125;
+__device__ __forceinline__ bool separated(double r0, double along, double limit) {
+  return along > 0.0 && along * along > kSeparation * kSeparation * limit * limit * r0;
+}
+__device__ __forceinline__ bool close_pair(const PairGeometry& p, double limit, double reach) {
+  if (p.r0 >= limit * limit) return false;
+  const double x = fmin(fmin(p.dgx0, p.dgx1), -(p.dgx0 + p.dgx1)),
+               y = fmax(fmax(p.dgy0, p.dgy1), -(p.dgy0 + p.dgy1));
+  return !separated(p.r0, fma(reach, x - y, p.r0), limit);
+}
+
+// Box of a cell's centroid and rR: the high words of its bounds, as integers of the same order
+// (two that compare equal may still meet).
+struct Box {
+  int lo[3], hi[3];
+};
+__device__ __forceinline__ Box cell_box(const Tile& t, int c) {
+  auto key = [](double x) {
+    const int b = __double2hiint(x);
+    return b ^ ((b >> 31) & 0x7fffffff);
+  };
+  const double r = t.G(rR, c);
+  Box b;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double x = t.G(rC + d, c);
+    b.lo[d] = key(x - r);
+    b.hi[d] = key(x + r);
+  }
+  return b;
+}
+// Box of a warp's tile of n cells.
+__device__ __forceinline__ Box tile_box(const Tile& t, int it, int n) {
+  Box b = cell_box(t, it);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    b.lo[d] = __reduce_min_sync(0xffffffffu, it < n ? b.lo[d] : 0x7fffffff);
+    b.hi[d] = __reduce_max_sync(0xffffffffu, it < n ? b.hi[d] : static_cast<int>(0x80000000));
+  }
+  return b;
+}
+// Trial cells (bit j) of [j0, j1) whose box meets that of the test tile: those that close_pair
+// has to look at.  Far tiles have none.
+__device__ __forceinline__ unsigned cells_in_reach(const Box& test, const Tile& S, int it, int j0,
+                                                   int j1) {
+  const Box b = cell_box(S, it);
+  bool meets = it >= j0 && it < j1;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) meets = meets && b.lo[d] <= test.hi[d] && b.hi[d] >= test.lo[d];
+  return __ballot_sync(0xffffffffu, meets);
+}
+
 // The 6-point rule: two orbits of three points on each cell.  The loop over the test
 // cell's orbits stays rolled (18 point pairs of straight code), everything else is in
 // registers.
@@ -314,17 +396,7 @@ __device__ __forceinline__ void pair_orbits(const PairGeometry& p, const Tile& T
       }
     }
   }
-#pragma unroll
-  for (int part = 0; part < NP; ++part) {
-    out.s[part] = 0.0;
-#pragma unroll
-    for (int a = 0; a < NBT; ++a)
-#pragma unroll
-      for (int b = 0; b < NBS; ++b) {
-        out.f[part][a][b] = 0.0;
-        if constexpr (PAIRED) out.t[part][a][b] = 0.0;
-      }
-  }
+  clear(out);
   // c-terms of the test basis (w phi_a = c + d [a = point]), added to every row at the end
   double cf[NP][NBS], ct[PAIRED ? NP : 1][NBS];
 #pragma unroll
@@ -565,10 +637,84 @@ __device__ __forceinline__ void point_block(const PairGeometry& p, double ex0, d
   }
 }
 
-// CTAs per SM the register allocation must allow.
+// A close pair: the squared distances from the components of
+// x_p - y_q = dc + alpha_p g_0 + beta_p g_1 - (alpha_q g'_0 + beta_q g'_1), test points first,
+// first + step, ...; phases not referenced to the pair (dc may be zero).  Adds to out.  Rolled
+// loops: these pairs are few.
+template <int KER, int OP, int NBT, int NBS, bool PAIRED>
+__device__ __forceinline__ void pair_by_components(
+    const PairGeometry& p, const Tile& T, int it, const Tile& S, int js, const double* rt, int Q,
+    int first, int step, double k,
+    Blocks<Traits<KER, OP, NBT, NBS, PAIRED>::kParts, NBT, NBS, PAIRED>& out) {
+  using Tr = Traits<KER, OP, NBT, NBS, PAIRED>;
+  constexpr int NP = Tr::kParts;
+#pragma unroll 1
+  for (int i = first; i < Q; i += step) {
+    const double* x = rt + kRuleStride * i;  // alpha, beta, w, w phi_0, w phi_1, w phi_2
+    double dx[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      dx[d] = ((T.G(rC + d, it) - S.G(rC + d, js)) + (T.G(rL + d, it) - S.G(rL + d, js))) +
+              fma(x[0], T.G(rG0 + d, it), x[1] * T.G(rG1 + d, it));
+    double U[NP][NBS], V[PAIRED ? NP : 1][NBS], G[NP];
+#pragma unroll
+    for (int part = 0; part < NP; ++part) {
+      G[part] = 0.0;
+#pragma unroll
+      for (int b = 0; b < NBS; ++b) {
+        U[part][b] = 0.0;
+        if constexpr (PAIRED) V[part][b] = 0.0;
+      }
+    }
+#pragma unroll 1
+    for (int q = 0; q < Q; ++q) {
+      const double* y = rt + kRuleStride * q;
+      double r2 = 0.0, K[2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double e = dx[d] - fma(y[0], S.G(rG0 + d, js), y[1] * S.G(rG1 + d, js));
+        r2 = fma(e, e, r2);
+      }
+      kernel_values<KER, OP, kAnyPhase, 1>(&r2, k, 0.0, K, K + 1);
+      const double fq = Tr::kTrialFactor ? fma(y[0], p.fy0, fma(y[1], p.fy1, p.fy)) : 1.0;
+#pragma unroll
+      for (int part = 0; part < NP; ++part) {
+        if constexpr (Tr::kHSSum) G[part] = fma(K[part], y[2], G[part]);
+        if constexpr (Tr::kBlock) {
+#pragma unroll
+          for (int b = 0; b < NBS; ++b) {
+            const double u = NBS == 3 ? y[3 + b] : y[2];
+            U[part][b] = fma(K[part], OP == kADL && !PAIRED ? u * fq : u, U[part][b]);
+            if constexpr (PAIRED) V[part][b] = fma(K[part], u * fq, V[part][b]);
+          }
+        }
+      }
+    }
+    const double ap = Tr::kTestFactor ? fma(x[0], p.fx0, fma(x[1], p.fx1, p.fx)) : 1.0;
+#pragma unroll
+    for (int part = 0; part < NP; ++part) {
+      if constexpr (Tr::kHSSum) out.s[part] = fma(x[2], G[part], out.s[part]);
+      if constexpr (Tr::kBlock) {
+#pragma unroll
+        for (int a = 0; a < NBT; ++a) {
+          const double c = NBT == 3 ? x[3 + a] : x[2];
+#pragma unroll
+          for (int b = 0; b < NBS; ++b) {
+            out.f[part][a][b] = fma(c, Tr::kTestFactor ? ap * U[part][b] : U[part][b], out.f[part][a][b]);
+            if constexpr (PAIRED) out.t[part][a][b] = fma(c, V[part][b], out.t[part][a][b]);
+          }
+        }
+      }
+    }
+  }
+}
+
+// CTAs per SM the register allocation must allow.  (Helmholtz DP0 x DP0: three; with four, 128
+// registers, the values that the close pairs need after the loop cost 3 %: 20,480 triangles,
+// k = 8, 13.12 ms against 12.76.)
 template <bool ORBITS, int KER, int OP, int NBT, int NBS, bool PAIRED>
 constexpr int min_ctas() {
-  if (KER == kHelmholtz) return PAIRED ? 2 : NBT * NBS == 9 ? 3 : NBS == 3 || NBT == 3 ? 3 : 4;
+  if (KER == kHelmholtz) return PAIRED ? 2 : 3;
   return PAIRED ? (ORBITS ? 3 : 2) : OP == kHS && ORBITS ? 4 : OP == kHS || NBT * NBS == 9 ? 3 : 4;
 }
 
@@ -613,7 +759,7 @@ __host__ __device__ inline Layout layout(int Q, int ns, int gather, int cap, int
   Layout l{};
   size_t o = 16;
   l.rule = o;
-  if (!ORBITS) o += sizeof(double) * kRuleStride * Q;
+  o += sizeof(double) * kRuleStride * Q;
   l.lengths = o;
   if (!ORBITS) o += sizeof(double) * static_cast<size_t>(ns) * ((Q + 1) & ~1);
   l.trial = o;
@@ -656,16 +802,17 @@ __device__ __forceinline__ Tile tile_at(unsigned char* at) {
 }
 
 // Issues the bulk copies of one tile (one thread): all geometry rows and the vertex ids.
-constexpr unsigned kStagedBytes = sizeof(double) * kRows * kTile + sizeof(int) * 3 * kTile;
+constexpr size_t kTileStride = sizeof(double) * kRows * kTile + sizeof(int) * 3 * kTile;  // in memory
+constexpr unsigned kStagedBytes = sizeof(double) * kNumGeomFields * kTile + sizeof(int) * 3 * kTile;
 __device__ inline void stage_geometry(const Tile& t, const CellSet& cs, int c0, uint64_t* m) {
   const int64_t S = cs.stride;
-  for (int f = 0; f < kRows; ++f)
+  for (int f = 0; f < kNumGeomFields; ++f)
     bulk_copy(t.geo + f * kTile, cs.geom + f * S + c0, sizeof(double) * kTile, m);
   for (int v = 0; v < 3; ++v) bulk_copy(t.vid + v * kTile, cs.vids + v * S + c0, sizeof(int) * kTile, m);
 }
 
-// The rows of column c as Row describes them.
-__device__ __forceinline__ void geometry_to_offsets(const Tile& t, int c) {
+// The rows of column c as Row describes them, for a rule of that reach (rR to about 20 bits).
+__device__ __forceinline__ void geometry_to_offsets(const Tile& t, int c, double reach) {
   double g0[3], g1[3], g2[3], e[3] = {0.0, 0.0, 0.0};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -684,12 +831,160 @@ __device__ __forceinline__ void geometry_to_offsets(const Tile& t, int c) {
     t.geo[(rG1 + d) * kTile + c] = g1[d];
     t.geo[(rE + d) * kTile + c] = e[d];
   }
+  const double most = fmax(fmax(e[0], e[1]), e[2]);
+  double root;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(root) : "d"(most));
+  t.geo[rR * kTile + c] = most > 0.0 ? reach * (1.0 / (1.0 - kSeparation)) * (most * root) : 0.0;
 }
 
 // Curl of basis function a of a flat cell from its offsets: t0 - t1, t1, -t0.
 __device__ __forceinline__ double curl_of(const Tile& t, int c, int a, int d) {
   const double g0 = t.G(rG0 + d, c), g1 = t.G(rG1 + d, c);
   return a == 0 ? fma(2.0, g1, g0) : a == 1 ? -(fma(2.0, g0, g1)) : g0 - g1;
+}
+
+// A pair's block from its sums: reference phase, jdet_x jdet_y / (4 pi), curls (Laplace
+// hypersingular: the sum s stays, the curls enter where it is added).
+template <int KER, int OP, int NBT, int NBS, bool PAIRED, int PH>
+__device__ __forceinline__ void finish_block(
+    const Tile& T, int it, const Tile& S, int js, double k, double kr0, double sc,
+    Blocks<Traits<KER, OP, NBT, NBS, PAIRED>::kParts, NBT, NBS, PAIRED>& blk) {
+  using Tr = Traits<KER, OP, NBT, NBS, PAIRED>;
+  constexpr int NP = Tr::kParts;
+  constexpr bool kC = NP == 2;
+  if constexpr (kC && PH != kAnyPhase) {
+    double ps, pc;
+    sincos_any(kr0, ps, pc);
+    if constexpr (Tr::kHSSum) {
+      const double re = blk.s[0] * pc - blk.s[1] * ps, im = blk.s[0] * ps + blk.s[1] * pc;
+      blk.s[0] = re;
+      blk.s[1] = im;
+    }
+    const double f = OP == kHS ? 1.0 : sc;
+    const double cr = pc * f, ci = ps * f;
+#pragma unroll
+    for (int a = 0; a < NBT; ++a)
+#pragma unroll
+      for (int b = 0; b < NBS; ++b) {
+        const double re = blk.f[0][a][b] * cr - blk.f[1][a][b] * ci;
+        blk.f[1][a][b] = blk.f[0][a][b] * ci + blk.f[1][a][b] * cr;
+        blk.f[0][a][b] = re;
+        if constexpr (PAIRED) {
+          const double tr = blk.t[0][a][b] * cr - blk.t[1][a][b] * ci;
+          blk.t[1][a][b] = blk.t[0][a][b] * ci + blk.t[1][a][b] * cr;
+          blk.t[0][a][b] = tr;
+        }
+      }
+  } else if constexpr (OP == kSL) {
+#pragma unroll
+    for (int part = 0; part < NP; ++part)
+#pragma unroll
+      for (int a = 0; a < NBT; ++a)
+#pragma unroll
+        for (int b = 0; b < NBS; ++b) blk.f[part][a][b] *= sc;
+  }
+  if constexpr (OP == kHS && kC) {
+    // curl-curl - k^2 normal-normal
+    const double nn = T.G(rN, it) * S.G(rN, js) + T.G(rN + 1, it) * S.G(rN + 1, js) +
+                      T.G(rN + 2, it) * S.G(rN + 2, js);
+    const double nnsc = -k * k * nn * sc;
+#pragma unroll
+    for (int a = 0; a < NBT; ++a)
+#pragma unroll
+      for (int b = 0; b < NBS; ++b) {
+        double cc = 0.0;
+        if constexpr (NBT == 3 && NBS == 3)
+#pragma unroll
+          for (int d = 0; d < 3; ++d) cc = fma(curl_of(T, it, a, d), curl_of(S, js, b, d), cc);
+        cc *= kInv4Pi;
+#pragma unroll
+        for (int part = 0; part < NP; ++part)
+          blk.f[part][a][b] = fma(nnsc, blk.f[part][a][b], blk.s[part] * cc);
+      }
+  }
+}
+
+// Adds a pair's block to the output (rows, cols: its global DOFs), and the transposed one
+// where the launch covers both orders of a pair.
+template <int KER, int OP, int NBT, int NBS, bool PAIRED>
+__device__ __forceinline__ void add_block(
+    const Tile& T, int it, const Tile& S, int js, const int* rows, const int* cols, double* out,
+    int64_t ld, bool mirror, int swapped,
+    Blocks<Traits<KER, OP, NBT, NBS, PAIRED>::kParts, NBT, NBS, PAIRED>& blk) {
+  constexpr int NP = Traits<KER, OP, NBT, NBS, PAIRED>::kParts;
+  if constexpr (KER == kLaplace && OP == kHS && NBT == 3 && NBS == 3) {
+#pragma unroll
+    for (int a = 0; a < NBT; ++a)
+#pragma unroll
+      for (int b = 0; b < NBS; ++b) {
+        double cc = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) cc = fma(curl_of(T, it, a, d), curl_of(S, js, b, d), cc);
+        blk.f[0][a][b] = blk.s[0] * cc * kInv4Pi;
+      }
+  }
+#pragma unroll
+  for (int b = 0; b < NBS; ++b) {
+    const int col = cols[b];
+#pragma unroll
+    for (int a = 0; a < NBT; ++a) {
+      const int64_t o = static_cast<int64_t>(col) * ld + rows[a];
+      const int64_t om = static_cast<int64_t>(rows[a]) * ld + col;
+#pragma unroll
+      for (int part = 0; part < NP; ++part) {
+        double v = blk.f[part][a][b], m = v;
+        if constexpr (PAIRED) {
+          m = swapped ? v : blk.t[part][a][b];
+          v = swapped ? blk.t[part][a][b] : v;
+        }
+        atomicAdd(out + NP * o + part, v);
+        if (mirror) atomicAdd(out + NP * om + part, m);
+      }
+    }
+  }
+}
+
+// The close pairs of a warp, after its other pairs: bit js of `todo` is the lane's pair with
+// trial cell js.  They are found before the loop over the pairs and added after it, directly:
+// with a branch for them in the loop everything was slower (20,480 triangles, Laplace
+// hypersingular P1 7.5 -> 8.0 ms, Helmholtz single layer DP0 12.7 -> 13.2; 80 triangles, 37-point
+// rule 21 -> 33 us); apart from it they cost 0 to 2 %.  tdofs, sdofs: DOFs of the tiles' cells.
+// DIRECT: the entries (and their transposes) were stored as zeros; SPLIT: sums[part][trial cell
+// of the chunk][lane] instead.
+template <int KER, int OP, int NBT, int NBS, bool DIRECT, bool PAIRED, bool SPLIT>
+__device__ __noinline__ void add_close_pairs(const Tile T, int it, const Tile S, unsigned todo,
+                                             const double* rt, int Q, int warp,
+                                             double k, const int* tdofs, const int* sdofs, int ti0,
+                                             int sj0, double* out, int64_t ld, bool mirror, int swapped,
+                                             double* sums, int ns, int j0) {
+  using Tr = Traits<KER, OP, NBT, NBS, PAIRED>;
+  constexpr int NP = Tr::kParts;
+  for (; todo; todo &= todo - 1) {
+    const int js = __ffs(todo) - 1;
+    const double sc = T.G(rJ, it) * S.G(rJ, js) * kInv4Pi;
+    PairGeometry p;
+    pair_geometry<KER, OP, NBT, NBS, PAIRED>(T, it, S, js, Tr::template kScaledFactors<kAnyPhase> ? sc : 1.0, p);
+    Blocks<NP, NBT, NBS, PAIRED> blk;
+    clear(blk);
+    pair_by_components<KER, OP, NBT, NBS, PAIRED>(p, T, it, S, js, rt, Q, SPLIT ? warp : 0,
+                                                  SPLIT ? kWarps : 1, k, blk);
+    finish_block<KER, OP, NBT, NBS, PAIRED, kAnyPhase>(T, it, S, js, k, 0.0, sc, blk);
+    if constexpr (DIRECT) {
+#pragma unroll
+      for (int part = 0; part < NP; ++part) {
+        const double v = blk.f[part][0][0];
+        if constexpr (SPLIT) {
+          sums[(part * ns + js - j0) * (kTile + 1) + it] = v;
+        } else {
+          out[NP * (static_cast<int64_t>(sj0 + js) * ld + ti0 + it) + part] = v;
+          if (mirror) out[NP * (static_cast<int64_t>(ti0 + it) * ld + sj0 + js) + part] = v;
+        }
+      }
+    } else {
+      add_block<KER, OP, NBT, NBS, PAIRED>(T, it, S, js, tdofs + it * NBT, sdofs + js * NBS, out, ld,
+                                           mirror, swapped, blk);
+    }
+  }
 }
 
 template <bool ORBITS, int KER, int OP, int NBT, int NBS, bool DIRECT, bool PAIRED, int PH,
@@ -823,7 +1118,19 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
       }
     }
   }
-  if constexpr (!ORBITS) {
+  if constexpr (ORBITS) {  // point a of orbit o is c + gamma_o g_a; constant indexes only
+    if (threadIdx.x < 6) {
+      const int a = threadIdx.x % 3;
+      const bool o = threadIdx.x >= 3;
+      const double g = o ? rule.g[1] : rule.g[0], c = o ? rule.c[1] : rule.c[0], d = o ? rule.d[1] : rule.d[0];
+      double* e = rt + threadIdx.x * kRuleStride;
+      e[0] = a == 0 ? g : a == 2 ? -g : 0.0;
+      e[1] = a == 1 ? g : a == 2 ? -g : 0.0;
+      e[2] = o ? rule.w[1] : rule.w[0];
+#pragma unroll
+      for (int b = 0; b < 3; ++b) e[3 + b] = a == b ? c + d : c;
+    }
+  } else {
     for (int i = threadIdx.x; i < Q; i += kThreads)
 #pragma unroll
       for (int f = 0; f < kPointFields; ++f) rt[i * kRuleStride + f] = rule.p[i][f];
@@ -836,13 +1143,16 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
     mbar_wait_bounded(mbar, 0);
     return;
   }
-  if (warp == 0) geometry_to_offsets(S, it);
+  if (warp == 0) geometry_to_offsets(S, it, rule.reach);
   if constexpr (SPLIT) {
-    if (warp == 1) geometry_to_offsets(T, it);
+    if (warp == 1) geometry_to_offsets(T, it, rule.reach);
   } else {
-    if (mine) geometry_to_offsets(T, it);
+    if (mine) geometry_to_offsets(T, it, rule.reach);
   }
+  Box box;
+  if (!SPLIT && mine) box = tile_box(T, it, nti);
   __syncthreads();
+  if (SPLIT) box = tile_box(T, it, nti);
   double* scurl = reinterpret_cast<double*>(smem + L.curls);  // [(b * 3 + d) * kTile + c]
   double* tcurl = stage + kSumBatch * kTile;                  // [(a * kTile + c) * 3 + d]
   if constexpr (kSumOnly && !DIRECT) {
@@ -870,12 +1180,21 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
   if (!mine && !SPLIT) return;  // SPLIT: the tile is the same for every warp
 
   const bool lane_cell = it < nti;
-  int a0 = -1, a1 = -2, a2 = -3;
-  if (lane_cell) {
-    a0 = T.vid[it];
-    a1 = T.vid[kTile + it];
-    a2 = T.vid[2 * kTile + it];
+  // the lane's pairs that the loop leaves out, bit js: vertex-sharing ones and close ones
+  unsigned skip = lane_cell ? 0u : ~0u, close = 0u;
+  if (same_grid && lane_cell) {
+    const int a0 = T.vid[it], a1 = T.vid[kTile + it], a2 = T.vid[2 * kTile + it];
+#pragma unroll 4
+    for (int js = j0; js < j1; ++js)
+      if (share_vertex(a0, a1, a2, S.vid[js], S.vid[kTile + js], S.vid[2 * kTile + js])) skip |= 1u << js;
   }
+  for (unsigned at = cells_in_reach(box, S, it, j0, j1); at; at &= at - 1) {
+    const int js = __ffs(at) - 1;
+    PairGeometry p;
+    pair_geometry<KER, kSL, 1, 1, false>(T, it, S, js, 1.0, p);
+    if (!((skip >> js) & 1u) && close_pair(p, T.G(rR, it) + S.G(rR, js), rule.reach)) close |= 1u << js;
+  }
+  skip |= close;
   int rows[NBT];  // direct adds: the lane's test DOFs
   if constexpr (!DIRECT) {
     if (!sh.gather)
@@ -912,32 +1231,17 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
 
 #pragma unroll 1
   for (int js = j0; js < j1; ++js) {
-    const bool have = lane_cell &&
-                      !(same_grid && share_vertex(a0, a1, a2, S.vid[js], S.vid[kTile + js],
-                                                  S.vid[2 * kTile + js]));
-    // jdet_x jdet_y / (4 pi); the normal factors carry it where the block is real
-    const double sc = T.G(rJ, it) * S.G(rJ, js) * kInv4Pi;
-    constexpr bool kScaledFactors = (Tr::kTestFactor || Tr::kTrialFactor) &&
-                                    (KER == kLaplace || PH == kAnyPhase);
+    const bool have = !((skip >> js) & 1u);
+    const double sc = T.G(rJ, it) * S.G(rJ, js) * kInv4Pi;  // jdet_x jdet_y / (4 pi)
     PairGeometry p;
-    pair_geometry<KER, OP, NBT, NBS, PAIRED>(T, it, S, js, kScaledFactors ? sc : 1.0, p);
+    pair_geometry<KER, OP, NBT, NBS, PAIRED>(T, it, S, js, Tr::template kScaledFactors<PH> ? sc : 1.0, p);
     double kr0 = 0.0;
     if constexpr (kC && PH != kAnyPhase) kr0 = k * (p.r0 * rsqrt_refined(p.r0));
     Blocks<NP, NBT, NBS, PAIRED> blk;
     if constexpr (ORBITS) {
       pair_orbits<KER, OP, NBT, NBS, PAIRED, PH>(p, T, it, S, js, rule, k, kr0, blk);
     } else {
-#pragma unroll
-      for (int part = 0; part < NP; ++part) {
-        blk.s[part] = 0.0;
-#pragma unroll
-        for (int a = 0; a < NBT; ++a)
-#pragma unroll
-          for (int b = 0; b < NBS; ++b) {
-            blk.f[part][a][b] = 0.0;
-            if constexpr (PAIRED) blk.t[part][a][b] = 0.0;
-          }
-      }
+      clear(blk);
       p.dgx0 *= 2.0;
       p.dgx1 *= 2.0;
       p.dgy0 *= -2.0;
@@ -960,57 +1264,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
       for (; rest < Q; rest += SPLIT ? kWarps : 1)
         point_block<KER, OP, NBT, NBS, PAIRED, PH, 1>(p, ex0, hx, ex1, rt, Yq, Q, rest, k, kr0, blk);
     }
-    // ---- the pair's block: reference phase, scale, curls
-    if constexpr (kC && PH != kAnyPhase) {
-      double ps, pc;
-      sincos_any(kr0, ps, pc);
-      if constexpr (Tr::kHSSum) {
-        const double re = blk.s[0] * pc - blk.s[1] * ps, im = blk.s[0] * ps + blk.s[1] * pc;
-        blk.s[0] = re;
-        blk.s[1] = im;
-      }
-      const double f = OP == kHS ? 1.0 : sc;
-      const double cr = pc * f, ci = ps * f;
-#pragma unroll
-      for (int a = 0; a < NBT; ++a)
-#pragma unroll
-        for (int b = 0; b < NBS; ++b) {
-          const double re = blk.f[0][a][b] * cr - blk.f[1][a][b] * ci;
-          blk.f[1][a][b] = blk.f[0][a][b] * ci + blk.f[1][a][b] * cr;
-          blk.f[0][a][b] = re;
-          if constexpr (PAIRED) {
-            const double tr = blk.t[0][a][b] * cr - blk.t[1][a][b] * ci;
-            blk.t[1][a][b] = blk.t[0][a][b] * ci + blk.t[1][a][b] * cr;
-            blk.t[0][a][b] = tr;
-          }
-        }
-    } else if constexpr (OP == kSL) {
-#pragma unroll
-      for (int part = 0; part < NP; ++part)
-#pragma unroll
-        for (int a = 0; a < NBT; ++a)
-#pragma unroll
-          for (int b = 0; b < NBS; ++b) blk.f[part][a][b] *= sc;
-    }
-    if constexpr (OP == kHS && kC) {
-      // curl-curl - k^2 normal-normal
-      const double nn = T.G(rN, it) * S.G(rN, js) + T.G(rN + 1, it) * S.G(rN + 1, js) +
-                        T.G(rN + 2, it) * S.G(rN + 2, js);
-      const double nnsc = -k * k * nn * sc;
-#pragma unroll
-      for (int a = 0; a < NBT; ++a)
-#pragma unroll
-        for (int b = 0; b < NBS; ++b) {
-          double cc = 0.0;
-          if constexpr (NBT == 3 && NBS == 3)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) cc = fma(curl_of(T, it, a, d), curl_of(S, js, b, d), cc);
-          cc *= kInv4Pi;
-#pragma unroll
-          for (int part = 0; part < NP; ++part)
-            blk.f[part][a][b] = fma(nnsc, blk.f[part][a][b], blk.s[part] * cc);
-        }
-    }
+    finish_block<KER, OP, NBT, NBS, PAIRED, PH>(T, it, S, js, k, kr0, sc, blk);
     // ---- where it goes
     if constexpr (DIRECT) {
       double v[2] = {have ? blk.f[0][0][0] : 0.0, kC && have ? blk.f[NP - 1][0][0] : 0.0};
@@ -1053,36 +1307,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
     } else if (!sh.gather) {
       // no accumulator: every lane adds its entries
       if (have) {
-        if constexpr (kSumOnly && NBT == 3 && NBS == 3) {
+        int cols[NBS];
 #pragma unroll
-          for (int a = 0; a < NBT; ++a)
-#pragma unroll
-            for (int b = 0; b < NBS; ++b) {
-              double cc = 0.0;
-#pragma unroll
-              for (int d = 0; d < 3; ++d) cc = fma(curl_of(T, it, a, d), curl_of(S, js, b, d), cc);
-              blk.f[0][a][b] = blk.s[0] * cc * kInv4Pi;
-            }
-        }
-#pragma unroll
-        for (int b = 0; b < NBS; ++b) {
-          const int col = S.ldof[b * kTile + js];
-#pragma unroll
-          for (int a = 0; a < NBT; ++a) {
-            const int64_t o = static_cast<int64_t>(col) * ld + rows[a];
-            const int64_t om = static_cast<int64_t>(rows[a]) * ld + col;
-#pragma unroll
-            for (int part = 0; part < NP; ++part) {
-              double v = blk.f[part][a][b], m = v;
-              if constexpr (PAIRED) {
-                m = swapped ? v : blk.t[part][a][b];
-                v = swapped ? blk.t[part][a][b] : v;
-              }
-              atomicAdd(out + NP * o + part, v);
-              if (mirror) atomicAdd(out + NP * om + part, m);
-            }
-          }
-        }
+        for (int b = 0; b < NBS; ++b) cols[b] = S.ldof[b * kTile + js];
+        add_block<KER, OP, NBT, NBS, PAIRED>(T, it, S, js, rows, cols, out, ld, mirror, swapped, blk);
       }
     } else if constexpr (NBT == 1) {
       // one DOF per test cell: lanes own their rows
@@ -1189,6 +1417,11 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
       }
     }
   }
+  if (__any_sync(0xffffffffu, close != 0u))
+    add_close_pairs<KER, OP, NBT, NBS, DIRECT, PAIRED, SPLIT>(
+        T, it, S, close, rt, Q, warp, k, DIRECT ? nullptr : tt.cell_dofs + static_cast<int64_t>(ti0) * NBT,
+        DIRECT ? nullptr : st.cell_dofs + static_cast<int64_t>(sj0) * NBS, ti0, sj0, out, ld, mirror,
+        swapped, mir, sh.ns, j0);
   // ---- flush
   if constexpr (DIRECT && SPLIT) {
     __syncthreads();
@@ -1248,8 +1481,18 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
 }
 
 // ---------------------------------------------------------------------- launches ---
+// The reach of a rule: with m the least barycentric coordinate of a point, the point is
+// c + sum_a (lambda_a - m) g_a, factors >= 0 whose sum is 1 - 3 m.
+inline double rule_reach(const RegularRule& r) {
+  double reach = 0.0;
+  for (int q = 0; q < r.npts; ++q)
+    reach = fmax(reach, 1.0 - 3.0 * fmin(fmin(r.phi[0][q], r.phi[1][q]), r.phi[2][q]));
+  return reach;
+}
+
 inline OrbitRule orbit_rule(const RegularRule& r) {
   OrbitRule o{};
+  o.reach = rule_reach(r);
   for (int i = 0; i < 2; ++i) {
     const double l0 = r.phi[0][3 * i];  // the orbit's first point is c + gamma g_0
     o.g[i] = (l0 - 1.0 / 3.0) * 1.5;
@@ -1266,6 +1509,7 @@ inline OrbitRule orbit_rule(const RegularRule& r) {
 inline PointRule point_rule(const RegularRule& r) {
   PointRule p{};
   p.npts = r.npts;
+  p.reach = rule_reach(r);
   for (int q = 0; q < r.npts; ++q) {
     const double l0 = r.phi[0][q], l1 = r.phi[1][q], l2 = r.phi[2][q];
     const double f[kPointFields] = {l0 - l2, l1 - l2, r.w[q], r.wphi[0][q], r.wphi[1][q], r.wphi[2][q]};

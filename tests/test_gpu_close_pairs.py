@@ -1,0 +1,67 @@
+"""Cells that nearly touch without sharing a vertex, against the oracle: two parallel sheets in
+one grid, turned so that no coordinate is exact, at gaps of 1e-2 to 1e-8 of a cell's edge, the
+rule points of facing cells opposite each other (equal sheets) or not (a coarse and a fine one).
+
+Tolerance: both sides form rule points with errors of a few eps |x|, so 1/r of facing points is
+off by up to 8 eps |x| / gap, 1/r^3 by three times that and the normal factor (x - y).n once
+more: 64 eps |x| / gap beside the parity tests' bound."""
+
+import numpy as np
+import pytest
+
+from ndgrid.grid import Grid
+
+from test_gpu_parity import FP64_TOL, OPS, SPACES, gpu_assemble, oracle_assemble, rel_err
+
+pytestmark = pytest.mark.gpu
+
+GAPS = [1e-2, 1e-4, 1e-6, 1e-8]
+
+
+def sheet(n):
+    x = np.linspace(0.0, 1.0, n + 1)
+    points = np.stack([np.repeat(x, n + 1), np.tile(x, n + 1), np.zeros((n + 1) ** 2)], axis=1)
+    a = (np.arange(n)[:, None] * (n + 1) + np.arange(n)[None, :]).ravel()
+    cells = np.stack([a, a + n + 1, a + 1, a + n + 1, a + n + 2, a + 1], axis=1).reshape(-1, 3)
+    return points, cells
+
+
+def turned(points):
+    q, _ = np.linalg.qr(np.random.default_rng(7).standard_normal((3, 3)))
+    return points @ q.T + np.array([0.1, -0.2, 0.3])
+
+
+def sheets(gap, n1=3, n2=3):
+    """Two sheets, `gap` edges (1 / n1) apart, and the tolerance."""
+    (p1, c1), (p2, c2) = sheet(n1), sheet(n2)
+    p2 = p2 + np.array([0.0, 0.0, gap / n1])
+    points = turned(np.vstack([p1, p2]))
+    size = np.abs(points).max()
+    tol = FP64_TOL + 64 * np.finfo(float).eps * size * n1 / gap
+    return Grid(points, np.vstack([c1, c2 + len(p1)])), tol
+
+
+@pytest.mark.parametrize("gap", GAPS)
+@pytest.mark.parametrize("q", [6, 16])
+@pytest.mark.parametrize("kernel,op,k,sp", [("laplace", "single_layer", 0.0, "dp0"),
+                                            ("laplace", "double_layer", 0.0, "p1"),
+                                            ("laplace", "adjoint_double_layer", 0.0, "dp1"),
+                                            ("laplace", "hypersingular", 0.0, "p1"),
+                                            ("helmholtz", "single_layer", 0.5, "dp0"),
+                                            ("helmholtz", "double_layer", 1.5, "p1"),
+                                            ("helmholtz", "adjoint_double_layer", 20.0, "p1"),
+                                            ("helmholtz", "hypersingular", 20.0, "p1")])
+def test_facing_sheets(gap, q, kernel, op, k, sp):
+    grid, tol = sheets(gap)
+    a = gpu_assemble(grid, kernel, op, k, SPACES[sp], q=q, one_space=True)
+    assert rel_err(a, oracle_assemble(grid, kernel, op, k, SPACES[sp], SPACES[sp], q=q)) <= tol
+
+
+@pytest.mark.parametrize("gap", GAPS)
+@pytest.mark.parametrize("kernel,op,k,test,trial", [("laplace", "single_layer", 0.0, "p1", "dp0"),
+                                                    ("laplace", "adjoint_double_layer", 0.0, "dp0", "p1"),
+                                                    ("helmholtz", "double_layer", 3.0, "dp0", "p1")])
+def test_coarse_against_fine_sheet(gap, kernel, op, k, test, trial):
+    grid, tol = sheets(gap, 1, 5)
+    a = gpu_assemble(grid, kernel, op, k, SPACES[test], SPACES[trial], q=37)
+    assert rel_err(a, oracle_assemble(grid, kernel, op, k, SPACES[test], SPACES[trial], q=37)) <= tol
