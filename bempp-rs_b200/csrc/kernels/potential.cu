@@ -14,7 +14,9 @@
 // cell's centroid c and offsets g_0, g_1 (regular_fp64.cuh): with dc = x - c,
 //   |x - y_q|^2 = (|dc|^2 + |y_q - c|^2) + alpha_q W0 + beta_q W1,  W = -2 dc.g,
 // three operations instead of six, (x - y_q).n = dc.n is formed once per cell, and the rule
-// points go through the kernel values six at a time.
+// points go through the kernel values six at a time.  Where those terms cancel (a point whose
+// distance from the centroid is below 1.14 times the rule points' largest: see
+// fp64::close_pair) the components of x - y_q are taken instead, after the other cells.
 //
 // Mapping.  A CTA stages one tile of 32 trial cells; each of its four warps has 32 points
 // (lane = point) and walks the tile's cells, or a chunk of them where the points are few.
@@ -97,6 +99,8 @@ __global__ void __launch_bounds__(kThreads, 4)
   __syncthreads();
   if (threadIdx.x < kTile) fp64::geometry_to_offsets(S, threadIdx.x, rule.reach);
   __syncthreads();
+  if (threadIdx.x < kTile)  // squared: compared with |x - c|^2
+    S.geo[fp64::rR * kTile + threadIdx.x] *= S.G(fp64::rR, threadIdx.x);
   for (int i = threadIdx.x; i < kTile * Q; i += kThreads) {
     const int c = i % kTile, q = i / kTile;
     const double al = ab[2 * q], be = ab[2 * q + 1];
@@ -118,6 +122,33 @@ __global__ void __launch_bounds__(kThreads, 4)
     for (int s = lane; s < nds * kTile * NP; s += 32) col[s] = 0.0;
     __syncwarp();
   }
+  // the cell's sums u, times sc, to the lane's entries
+  auto put = [&](int js, double (&u)[NP][NB], double sc) {
+    if (NB == 1) {
+      if (valid) {
+        const int64_t o = i + ld * dof[js];
+        if (NP == 2)
+          reinterpret_cast<double2*>(out)[o] = make_double2(u[0][0] * sc, u[NP - 1][0] * sc);
+        else
+          out[o] = u[0][0] * sc;
+      }
+    } else if (cap > 0) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        double* c = col + dof[js * NB + b] + lane;
+#pragma unroll
+        for (int part = 0; part < NP; ++part) c[part * kTile] = fma(u[part][b], sc, c[part * kTile]);
+      }
+    } else if (valid) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const int64_t o = i + ld * dof[js * NB + b];
+#pragma unroll
+        for (int part = 0; part < NP; ++part) atomicAdd(out + NP * o + part, u[part][b] * sc);
+      }
+    }
+  };
+  unsigned close = 0u;  // the lane's cells left for the second loop
   for (int js = j0; js < j1; ++js) {
     const double dx = (x0 - S.G(fp64::rC, js)) - S.G(fp64::rL, js),
                  dy = (x1 - S.G(fp64::rC + 1, js)) - S.G(fp64::rL + 1, js),
@@ -155,29 +186,40 @@ __global__ void __launch_bounds__(kThreads, 4)
     if (q < Q) some(q, std::integral_constant<int, 1>{});
     double sc = S.G(fp64::rJ, js) * kInv4Pi;
     if (OP == kDL) sc *= dot(fp64::rN);
-    if (NB == 1) {
-      if (valid) {
-        const int64_t o = i + ld * dof[js];
-        if (NP == 2)
-          reinterpret_cast<double2*>(out)[o] = make_double2(u[0][0] * sc, u[NP - 1][0] * sc);
-        else
-          out[o] = u[0][0] * sc;
-      }
-    } else if (cap > 0) {
+    // high words: no operation of the FP64 pipe, no branch before the kernel values
+    const bool near_cell = __double2hiint(r0) <= __double2hiint(S.G(fp64::rR, js));
+    close |= near_cell ? 1u << js : 0u;
+    if (!near_cell) put(js, u, sc);
+  }
+  if (!valid) close = 0u;
+  for (; close; close &= close - 1) {
+    const int js = __ffs(close) - 1;
+    const double dx = (x0 - S.G(fp64::rC, js)) - S.G(fp64::rL, js),
+                 dy = (x1 - S.G(fp64::rC + 1, js)) - S.G(fp64::rL + 1, js),
+                 dz = (x2 - S.G(fp64::rC + 2, js)) - S.G(fp64::rL + 2, js);
+    double u[NP][NB];
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        double* c = col + dof[js * NB + b] + lane;
+    for (int part = 0; part < NP; ++part)
 #pragma unroll
-        for (int part = 0; part < NP; ++part) c[part * kTile] = fma(u[part][b], sc, c[part * kTile]);
-      }
-    } else if (valid) {
+      for (int b = 0; b < NB; ++b) u[part][b] = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < Q; ++q) {
+      const double al = ab[2 * q], be = ab[2 * q + 1];
+      const double ex = dx - fma(al, S.G(fp64::rG0, js), be * S.G(fp64::rG1, js)),
+                   ey = dy - fma(al, S.G(fp64::rG0 + 1, js), be * S.G(fp64::rG1 + 1, js)),
+                   ez = dz - fma(al, S.G(fp64::rG0 + 2, js), be * S.G(fp64::rG1 + 2, js));
+      const double r2 = fma(ez, ez, fma(ey, ey, ex * ex));
+      double K[2];
+      fp64::kernel_values<KER, OP, fp64::kAnyPhase, 1>(&r2, k, 0.0, K, K + 1);
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const int64_t o = i + ld * dof[js * NB + b];
+      for (int b = 0; b < NB; ++b)
 #pragma unroll
-        for (int part = 0; part < NP; ++part) atomicAdd(out + NP * o + part, u[part][b] * sc);
-      }
+        for (int part = 0; part < NP; ++part) u[part][b] = fma(K[part], wt[q * NB + b], u[part][b]);
     }
+    double sc = S.G(fp64::rJ, js) * kInv4Pi;
+    if (OP == kDL)
+      sc *= fma(dz, S.G(fp64::rN + 2, js), fma(dy, S.G(fp64::rN + 1, js), dx * S.G(fp64::rN, js)));
+    put(js, u, sc);
   }
   if (NB > 1 && cap > 0 && valid) {
     // columns of DOFs that the chunk's cells do not touch stay zero

@@ -9,7 +9,14 @@ more: 64 eps |x| / gap beside the parity tests' bound."""
 import numpy as np
 import pytest
 
+from bempp.assembly.boundary import BoundaryAssemblerOptions
+from bempp.assembly.potential import (create_helmholtz_potential_assembler,
+                                      create_laplace_potential_assembler)
+from bempp.function_space import function_space
+from ndelement.ciarlet import Continuity, Family, create_family
+from ndelement.reference_cell import ReferenceCellType
 from ndgrid.grid import Grid
+from oracle import oracle, potential
 
 from test_gpu_parity import FP64_TOL, OPS, SPACES, gpu_assemble, oracle_assemble, rel_err
 
@@ -65,3 +72,30 @@ def test_coarse_against_fine_sheet(gap, kernel, op, k, test, trial):
     grid, tol = sheets(gap, 1, 5)
     a = gpu_assemble(grid, kernel, op, k, SPACES[test], SPACES[trial], q=37)
     assert rel_err(a, oracle_assemble(grid, kernel, op, k, SPACES[test], SPACES[trial], q=37)) <= tol
+
+
+@pytest.mark.parametrize("gap", GAPS)
+@pytest.mark.parametrize("q", [6, 16])
+@pytest.mark.parametrize("kernel,op,k,degree", [("laplace", "single_layer", 0.0, 0),
+                                                ("laplace", "double_layer", 0.0, 1),
+                                                ("helmholtz", "single_layer", 2.0, 2),
+                                                ("helmholtz", "double_layer", 2.0, 1)])
+def test_potential_above_a_sheet(gap, q, kernel, op, k, degree):
+    """Points `gap` edges above the rule points of a sheet's cells."""
+    n = 3
+    p, c = sheet(n)
+    x, _ = oracle.simplex_rule(q)
+    v = p[c]
+    above = (v[:, :1] + x[:, :1] * (v[:, 1:2] - v[:, :1]) + x[:, 1:] * (v[:, 2:] - v[:, :1])).reshape(-1, 3)
+    above = turned(above + np.array([0.0, 0.0, gap / n]))
+    points = turned(p)
+    opts = BoundaryAssemblerOptions()
+    opts.set_regular_quadrature_degree(ReferenceCellType.Triangle, q)
+    a = (create_laplace_potential_assembler(OPS[op], opts) if kernel == "laplace"
+         else create_helmholtz_potential_assembler(OPS[op], k, opts))
+    space = function_space(Grid(points, c), create_family(
+        Family.Lagrange, degree, Continuity.Standard if degree else Continuity.Discontinuous))
+    o = potential.potential(above, points, c.astype(np.int64), kernel, op, k=k, degree=degree,
+                            continuous=degree > 0, q_regular=q)
+    tol = FP64_TOL + 64 * np.finfo(float).eps * np.abs(above).max() * n / gap
+    assert rel_err(a.assemble(space, above), o) <= tol
