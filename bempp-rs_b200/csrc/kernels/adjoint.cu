@@ -356,12 +356,16 @@ __global__ void __launch_bounds__(kThreads, 3)
 // coefficients: row sums R_p = sum_q w_q h_pq, column sums, and G_pb = sum over the trial
 // orbits of w gamma h.  So the loop over point pairs keeps scalars (about 5 operations per
 // pair for all sums, where accumulating the vectors per test and per trial point took 8 and
-// the differences 3 more) and the vectors are formed once per cell pair.
+// the differences 3 more) and the vectors are formed once per cell pair.  Pairs nearly in
+// contact (close_pair; the combinations above lose eps H / r there, as differences of
+// coordinates do) are left to a second pass, CLOSE, that takes the squared distances from the
+// components of x_p - y_q: in one loop with the others they cost 200 bytes of spills.
+// Returns whether the lane has such pairs.
 // The largest circumradii of the two tiles decide between the phase referenced to the pair and
 // the reduced phase.  5,120 triangles, k = 5, B200: 3.3 ms with coordinate differences,
 // 1.97 in this form.
-template <int PH>
-__device__ __forceinline__ void adjoint_orbit_pairs(
+template <int PH, bool CLOSE>
+__device__ __forceinline__ bool adjoint_orbit_pairs(
     const Tile& T, const Tile& S, int it, int warp, int ti0, int sj0, int nti, int nsj, bool both,
     const fp64::OrbitRule& rule, double k, const double2* __restrict__ lam,
     const double2* __restrict__ mu, const double* jx, const double* jy, double* s_test,
@@ -372,10 +376,17 @@ __device__ __forceinline__ void adjoint_orbit_pairs(
   const double2 mi = valid && both ? mu[ti0 + it] : make_double2(0.0, 0.0);
   const int a0 = T.vid[it], a1 = T.vid[kTile + it], a2 = T.vid[2 * kTile + it];
   double* mine = s_test + warp * 9 * kTile + it;
+  bool found = false;
 #pragma unroll 1
   for (int js = warp; js < nsj; js += kWarps) {
-    const bool active = valid && !share_vertex(a0, a1, a2, S.vid[js], S.vid[kTile + js],
-                                               S.vid[2 * kTile + js]);
+    const bool regular = valid && !share_vertex(a0, a1, a2, S.vid[js], S.vid[kTile + js],
+                                                S.vid[2 * kTile + js]);
+    PairGeometry p;
+    pair_geometry<kHelmholtz, kSL, 1, 1, false>(T, it, S, js, 1.0, p);
+    const bool close = regular && close_pair(p, T.G(rR, it) + S.G(rR, js), rule.reach);
+    const bool active = CLOSE ? close : regular && !close;
+    found = found || close;
+    if (CLOSE && !__any_sync(0xffffffffu, active)) continue;
     // c = conj(lambda_i) mu_j (+ conj(lambda_j) mu_i off the diagonal)
     const double2 mj = mu[sj0 + js];
     double c_re = li.x * mj.x + li.y * mj.y, c_im = li.x * mj.y - li.y * mj.x;
@@ -384,8 +395,6 @@ __device__ __forceinline__ void adjoint_orbit_pairs(
       c_re += lj.x * mi.x + lj.y * mi.y;
       c_im += lj.x * mi.y - lj.y * mi.x;
     }
-    PairGeometry p;
-    pair_geometry<kHelmholtz, kSL, 1, 1, false>(T, it, S, js, 1.0, p);
     // phase referenced to the pair: c is rotated by e^{ik r0} for the gradient terms, the
     // sums S0, Sk after the loop
     double kr0 = 0.0, pc = 1.0, ps = 0.0, q_re = c_re, q_im = c_im;
@@ -435,6 +444,21 @@ __device__ __forceinline__ void adjoint_orbit_pairs(
           for (int i = 0; i < 6; ++i) r2[i] = X + Y[i / 3][i % 3];
 #pragma unroll
           for (int i = 0; i < 6; ++i) r2[i] = fma(i < 3 ? m0 : m1, M[a][i % 3], r2[i]);
+          if (CLOSE) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) r2[i] = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const double g0 = T.G(rG0 + d, it), g1 = T.G(rG1 + d, it), u0 = S.G(rG0 + d, js), u1 = S.G(rG1 + d, js);
+              const double x = fma(gp, a == 0 ? g0 : a == 1 ? g1 : -(g0 + g1),
+                                   (T.G(rC + d, it) - S.G(rC + d, js)) + (T.G(rL + d, it) - S.G(rL + d, js)));
+#pragma unroll
+              for (int i = 0; i < 6; ++i) {
+                const double e = fma(-rule.g[i / 3], i % 3 == 0 ? u0 : i % 3 == 1 ? u1 : -(u0 + u1), x);
+                r2[i] = fma(e, e, r2[i]);
+              }
+            }
+          }
 #pragma unroll
           for (int i = 0; i < 6; ++i) y[i] = rsqrt_refined(r2[i]);
 #pragma unroll
@@ -557,6 +581,7 @@ __device__ __forceinline__ void adjoint_orbit_pairs(
     if ((it & 3) == 0) s_trial[js * 9 + (it >> 2)] += v1;  // each js belongs to one warp
     if (it == 1) s_trial[js * 9 + 8] += v8;
   }
+  return found;
 }
 
 __global__ void __launch_bounds__(kThreads, 2)
@@ -626,12 +651,14 @@ __global__ void __launch_bounds__(kThreads, 2)
   __syncthreads();
 
   double jval = 0.0, dk = 0.0;
-  if (referenced)
-    adjoint_orbit_pairs<kReferenced>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k, lam, mu, jx,
-                                     jy, s_test, s_trial, jval, dk);
-  else
-    adjoint_orbit_pairs<kAnyPhase>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k, lam, mu, jx,
-                                   jy, s_test, s_trial, jval, dk);
+  const bool found =
+      referenced ? adjoint_orbit_pairs<kReferenced, false>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k,
+                                                           lam, mu, jx, jy, s_test, s_trial, jval, dk)
+                 : adjoint_orbit_pairs<kAnyPhase, false>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k,
+                                                         lam, mu, jx, jy, s_test, s_trial, jval, dk);
+  if (__any_sync(0xffffffffu, found))
+    adjoint_orbit_pairs<kAnyPhase, true>(T, S, it, warp, ti0, sj0, nti, nsj, both, rule, k, lam, mu, jx,
+                                         jy, s_test, s_trial, jval, dk);
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) {
     jval += __shfl_xor_sync(0xffffffffu, jval, s);

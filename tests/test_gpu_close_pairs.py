@@ -99,3 +99,39 @@ def test_potential_above_a_sheet(gap, q, kernel, op, k, degree):
                             continuous=degree > 0, q_regular=q)
     tol = FP64_TOL + 64 * np.finfo(float).eps * np.abs(above).max() * n / gap
     assert rel_err(a.assemble(space, above), o) <= tol
+
+
+@pytest.mark.parametrize("gap", GAPS[:3])
+@pytest.mark.parametrize("k", [0.5, 20.0])
+@pytest.mark.parametrize("q", [6, 16])
+def test_gradient_between_sheets(gap, k, q):
+    """lambda lives on one sheet and mu on the other, so that only facing pairs count.  Against
+    the rule's sum differentiated by torch: grad 1/r loses as the double layer does."""
+    import torch
+
+    from bempp.autograd import energy_and_gradient
+
+    grid, tol = sheets(gap)
+    points, cells = np.array(grid.points), np.array(grid.cells, dtype=np.int64)
+    n = len(cells) // 2
+    rng = np.random.default_rng(3)
+    lam, mu = (rng.standard_normal(2 * n) + 1j * rng.standard_normal(2 * n) for _ in range(2))
+    lam[n:] = 0.0
+    mu[:n] = 0.0
+    j, dk, grad = energy_and_gradient(points, cells, k, lam, mu, regular_points=q)
+    xi, w = oracle.simplex_rule(q)
+    phi = torch.tensor(np.stack([1.0 - xi.sum(1), xi[:, 0], xi[:, 1]], axis=1))
+    w = torch.tensor(w)
+    p = torch.tensor(points, requires_grad=True)
+    kt = torch.tensor(k, dtype=torch.float64, requires_grad=True)
+    v = p[torch.tensor(cells)]
+    jdet = torch.linalg.norm(torch.linalg.cross(v[:, 1] - v[:, 0], v[:, 2] - v[:, 0]), dim=1)
+    x = torch.einsum("qa,cad->cqd", phi, v)
+    r = torch.linalg.norm(x[:n, None, :, None] - x[None, n:, None, :], dim=-1)
+    a = torch.einsum("ijpq,p,q->ij", torch.polar(1.0 / r, kt * r), w.cdouble(), w.cdouble())
+    a = a * jdet[:n, None] * jdet[None, n:] / (4 * np.pi)
+    value = (torch.tensor(lam[:n]).conj() @ a @ torch.tensor(mu[n:])).real
+    value.backward()
+    assert abs(j.item() - value.item()) <= tol * max(abs(value.item()), a.abs().max().item())
+    assert np.abs(grad.cpu().numpy() - p.grad.numpy()).max() <= tol * p.grad.abs().max().item()
+    assert abs(dk.item() - kt.grad.item()) <= tol * max(abs(kt.grad.item()), 1.0)
