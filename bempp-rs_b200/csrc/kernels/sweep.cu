@@ -42,6 +42,10 @@ using namespace tiles;
 constexpr int kPass = 8;          // wavenumbers per pass over a tile pair
 constexpr int kMoments = 12;      // at most: 9 for |t| <= 0.8, 12 for |t| <= 2
 constexpr float kWide = 2.0f;     // the moments' largest |x t|
+// The moments' largest |t|: t^11 <= 7e19 stays within FP32, and where x^11 underflows, (x t)^11
+// is below rounding.  A pass with a wavenumber beyond it takes the phases of each on its own, so
+// that no wavenumber spoils another's matrix.
+constexpr float kMomentRange = 64.0f;
 constexpr int kMirrorRow = 36;    // padded row of the transposing buffer: no bank conflicts
 constexpr int kMirrorGroup = 4;   // trial cells per group of the transposing buffer
 constexpr int kSingularGroup = 4; // wavenumbers per thread of the vertex-sharing pairs
@@ -76,7 +80,7 @@ __device__ inline void fill_table(PassTable& p, const double* __restrict__ ks, i
   double K = 0.0;
   for (int i = 0; i < n; ++i) {
     const double m = fabs(__ldg(ks + i));
-    if (m <= 1e30) K = fmax(K, m);  // one beyond FP32's range spoils its own matrix only
+    if (m <= 1e30) K = fmax(K, m);  // one beyond FP32's range has no part in the scale
   }
   if (K < 1e-20) K = 0.0;
   const float Kf = K > 0.0 ? static_cast<float>(K) : 1e-20f;
@@ -324,7 +328,8 @@ __global__ void __launch_bounds__(kThreads, 4)
               continue;
             }
             // every wavenumber is taken by one of the two (a NaN by both)
-            if (reach * table.least <= kWide) by_moments(std::integral_constant<int, kMoments>{});
+            const bool moments = top <= kMomentRange;
+            if (moments && reach * table.least <= kWide) by_moments(std::integral_constant<int, kMoments>{});
             if (!(top <= kWide)) {
               float2 f[18], t[18];
               int at = 0;
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll 1
               for (int kk = 0; kk < nk; ++kk) {
                 const float2 x = f2(table.x[kk]);
-                if (reach * fabsf(x.x) <= kWide) continue;  // warp-uniform: done above
+                if (moments && reach * fabsf(x.x) <= kWide) continue;  // warp-uniform: done above
                 float re = 0.f, im = 0.f, cre = 0.f, cim = 0.f;
 #pragma unroll
                 for (int g = 0; g < 18; g += 3) {
