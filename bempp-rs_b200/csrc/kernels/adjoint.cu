@@ -858,9 +858,9 @@ cudaError_t launch_adjoint_sl(const CellSet& cs, const RegularRule& rule,
     adjoint_sl_orbits<<<grid, kThreads, bytes, stream>>>(cs, fp64::orbit_rule(rule), k, l2, m2,
                                                          grad_cell, totals, timeouts, polls);
   } else {
-    auto fn = rule.npts == 6 ? adjoint_sl_regular<6, true>
-              : mixed        ? adjoint_sl_regular<0, true>
-                             : adjoint_sl_regular<0, false>;
+    auto fn = !mixed           ? adjoint_sl_regular<0, false>
+              : rule.npts == 6 ? adjoint_sl_regular<6, true>
+                               : adjoint_sl_regular<0, true>;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     fn<<<grid, kThreads, smem, stream>>>(cs, rule, k, l2, m2, grad_cell, totals, timeouts, polls);
   }
