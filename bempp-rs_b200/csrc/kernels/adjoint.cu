@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 3)
         phase_cos_sin(k * r0, pc, ps);
         const float cr = static_cast<float>(c_re * pc - c_im * ps);
         const float ci = static_cast<float>(c_re * ps + c_im * pc);
-        const bool taylor = k * (T.G(fRad, it) + S.G(fRad, js)) <= 0.8;
+        const bool taylor = fabs(k) * (T.G(fRad, it) + S.G(fRad, js)) <= 0.8;
         float fS0r = 0.f, fS0i = 0.f, fSkr = 0.f, fSki = 0.f;
         float fuq[QT > 0 ? QT : kMaxRegularPoints][3];
         float fvt[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       // e^{ikr} referenced to the pair (e^{ik r0} e^{ik (r - r0)}, r0 = |c_x - c_y|) when
       // k (rad_x + rad_y) <= 0.8 bounds every phase k (r - r0): c is rotated by e^{ik r0}
       // for the gradient terms and the sums S0, Sk are rotated back after the loop
-      const bool ref = k * (T.G(fRad, it) + S.G(fRad, js)) <= 0.8;
+      const bool ref = fabs(k) * (T.G(fRad, it) + S.G(fRad, js)) <= 0.8;
       double kr0 = 0.0, pc = 1.0, ps = 0.0, cq_re = c_re, cq_im = c_im;
       if (ref) {
         const double dcx = T.G(fCx, it) - S.G(fCx, js), dcy = T.G(fCy, it) - S.G(fCy, js),

@@ -744,7 +744,7 @@ __device__ __forceinline__ void block_fp32(const Tile& T, int it, const Tile& S,
     phase_cos_sin(k * r0, ph_c, ph_s);
     // warp-uniform choice, so that a warp never runs two variants
     if (PH == kPhaseRuntime) {
-      const double bound = k * (T.G(fRad, it) + S.G(fRad, js));
+      const double bound = fabs(k) * (T.G(fRad, it) + S.G(fRad, js));
       const unsigned active = __activemask();
       small_phase = __all_sync(active, bound <= static_cast<double>(kSmallPhaseMax));
       wide_phase = __all_sync(active, bound <= static_cast<double>(kWidePhaseMax));

@@ -388,15 +388,14 @@ __global__ void __launch_bounds__(kThreads, 4)
 
 // Single-layer DP0 entry of one cell pair (test i, trial j) by the 6-point rule in FP64,
 // points and geometry from the grid arrays: phase referenced to the pair when
-// k (rad_i + rad_j) <= 0.8, else sincos_cw.
+// |k| (rad_i + rad_j) <= 0.8, else sincos_cw.
 __device__ double2 sl_dp0_pair_fp64(const CellSet& cs, int i, int j, const RegularRule& rule,
                                     double k) {
   const int64_t S = cs.stride;
   const double dcx = g(cs.geom, kCx, cs.stride, i) - g(cs.geom, kCx, cs.stride, j);
   const double dcy = g(cs.geom, kCy, cs.stride, i) - g(cs.geom, kCy, cs.stride, j);
   const double dcz = g(cs.geom, kCz, cs.stride, i) - g(cs.geom, kCz, cs.stride, j);
-  const bool ref = k * (g(cs.geom, kRad, cs.stride, i) + g(cs.geom, kRad, cs.stride, j)) <=
-                   0.8;
+  const bool ref = fabs(k) * (g(cs.geom, kRad, cs.stride, i) + g(cs.geom, kRad, cs.stride, j)) <= 0.8;
   double kr0 = 0.0, pc = 1.0, ps = 0.0;
   if (ref) {
     const double r0sq = dcx * dcx + dcy * dcy + dcz * dcz;
