@@ -156,23 +156,23 @@ __device__ __forceinline__ void sincos_taylor(double r, double& sr, double& cr) 
 
 // sin(t) and cos(t) in FP64 for |t| <= 0.8 (pair-referenced phases k (r - r0) of the
 // FP64 regular kernels): cos t = 1 + z P(z), sin t = t + t z Q(z), z = t^2, with P and Q of
-// degree 5 from a near-minimax fit at 50 digits (fit_phase_polys.py fp64); max abs
-// errors 2.5e-16 (cos) and 1.9e-17 (sin) on |t| <= 0.8.
+// degree 5, minimax in the cosine and sine themselves (fit_phase_polys.py fp64); max abs
+// errors 8.2e-17 (cos) and 7.9e-18 (sin) on |t| <= 0.8 before the rounding of the evaluation.
 __device__ __forceinline__ void sincos_small(double t, double& s, double& c) {
   const double z = t * t;
-  double p = 2.0657616391477202e-09;
-  p = fma(p, z, -2.755574396426964e-07);
-  p = fma(p, z, 2.4801582078024058e-05);
-  p = fma(p, z, -0.0013888888881056654);
-  p = fma(p, z, 0.04166666666662371);
-  p = fma(p, z, -0.4999999999999996);
+  double p = 2.0624516558338953e-09;
+  p = fma(p, z, -2.755514230336705e-07);
+  p = fma(p, z, 2.4801578051260594e-05);
+  p = fma(p, z, -0.0013888888869009524);
+  p = fma(p, z, 0.041666666666470224);
+  p = fma(p, z, -0.49999999999999356);
   c = fma(z, p, 1.0);
-  double q = 1.5912864224903485e-10;
-  q = fma(q, z, -2.5051057394492127e-08);
-  q = fma(q, z, 2.7557315738586845e-06);
-  q = fma(q, z, -0.00019841269836043575);
-  q = fma(q, z, 0.008333333333330467);
-  q = fma(q, z, -0.16666666666666663);
+  double q = 1.5882222316304609e-10;
+  q = fma(q, z, -2.505048532825731e-08);
+  q = fma(q, z, 2.755731176635098e-06);
+  q = fma(q, z, -0.00019841269823504595);
+  q = fma(q, z, 0.00833333333331308);
+  q = fma(q, z, -0.16666666666666585);
   s = t * fma(z, q, 1.0);
 }
 
@@ -196,15 +196,15 @@ __device__ __forceinline__ void sincos_cw(double t, double& s, double& c) {
 template <int N, bool SHORT = false>
 __device__ __forceinline__ void sincos_small_n(const double t[N], double s[N], double c[N]) {
   constexpr int kTerms = SHORT ? 5 : 6;
-  // |t| <= 0.42: interpolation of the two series at Chebyshev points, errors 1.2e-16, 4e-18
-  constexpr double P5[5] = {-2.746539758703359e-07, 2.4801445491762405e-05, -0.0013888888799568808,
-                            0.04166666666646974, -0.4999999999999993};
-  constexpr double Q5[5] = {-2.4981384587602678e-08, 2.7557210109293225e-06, -0.00019841269772540994,
-                            0.00833333333331818, -0.1666666666666666};
-  constexpr double P6[6] = {2.0657616391477202e-09,  -2.755574396426964e-07, 2.4801582078024058e-05,
-                           -0.0013888888881056654, 0.04166666666662371,    -0.4999999999999996};
-  constexpr double Q6[6] = {1.5912864224903485e-10, -2.5051057394492127e-08, 2.7557315738586845e-06,
-                           -0.00019841269836043575, 0.008333333333330467,   -0.16666666666666663};
+  // |t| <= 0.42: degree 4 (fit_phase_polys.py fp64 0.42 4), errors 3.4e-17, 1.2e-18
+  constexpr double P5[5] = {-2.7448953184516356e-07, 2.480137779423873e-05, -0.0013888888704968658,
+                            0.041666666665961964, -0.49999999999999123};
+  constexpr double Q5[5] = {-2.496406062758246e-08, 2.755713667264e-06, -0.000198412696653988,
+                            0.008333333333256544, -0.1666666666666655};
+  constexpr double P6[6] = {2.0624516558338953e-09,  -2.755514230336705e-07, 2.4801578051260594e-05,
+                           -0.0013888888869009524, 0.041666666666470224,    -0.49999999999999356};
+  constexpr double Q6[6] = {1.5882222316304609e-10, -2.505048532825731e-08, 2.755731176635098e-06,
+                           -0.00019841269823504595, 0.00833333333331308,   -0.16666666666666585};
   double z[N], p[N], q[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) z[i] = t[i] * t[i];
@@ -229,7 +229,7 @@ __device__ __forceinline__ void sincos_small_n(const double t[N], double s[N], d
 // sin(t), cos(t) of N arguments of any size: reduction by pi/2 (the multiple read from the
 // low word of t (2/pi) + 1.5 2^52, two-part pi/2, each step one FMA), sincos_small_n, the
 // quadrant's exchange by integer operations.  18 FP64 operations; absolute error about
-// 2.5e-16.  Finite arguments from 2^51 on (whose last digit is worth 0.5 or more, so that the
+// 1.5e-16.  Finite arguments from 2^51 on (whose last digit is worth 0.5 or more, so that the
 // phase is arbitrary) are taken as 0 by a selection, so that the result is a point of the unit
 // circle; infinities and NaN give NaN.  A branch to a loop for them cut the N chains apart (Helmholtz double layer P1 of
 // 5,120 triangles, k = 8, on a B200: 2.80 ms with it, 2.65 without).

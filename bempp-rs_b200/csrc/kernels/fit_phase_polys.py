@@ -14,12 +14,13 @@ k (max rad_x + max rad_y) <= 0.8 and, after a reduction by pi/2, by every other 
 
 FP64 (sincos_small in common.cuh, the pair-referenced phases of the FP64 kernels):
 
-    python fit_phase_polys.py fp64
+    python fit_phase_polys.py fp64 [tmax degree]
 
-cos t ~ 1 + z P(z) and sin t ~ t + t z Q(z), z = t^2, P and Q of degree 5 on |t| <= 0.8,
-by Chebyshev interpolation of (cos(sqrt z) - 1) / z and (sin(sqrt z) / sqrt z - 1) / z on
-[0, 0.64] at 50 digits (mpmath.chebyfit, near-minimax); the script prints the
-coefficients rounded to double and the max errors of cos and sin with them.
+cos t ~ 1 + z P(z) and sin t ~ t + t z Q(z), z = t^2, P and Q of degree 5 on |t| <= 0.8
+(default) or of the given degree on |t| <= tmax, minimax in the errors of cos and sin (Remez
+exchange at 50 digits; an interpolation of P and Q at Chebyshev points has three times the
+error); the script prints the coefficients rounded to double and the max errors of cos and
+sin with them.
 """
 
 import numpy as np
@@ -65,6 +66,46 @@ def fit(tmax, ncos, nsin):
     return c, ec, s, es
 
 
+def remez(f, phi, n, zmax):
+    """Coefficients c that minimise max |f(z) - sum_j c_j phi(j, z)| on (0, zmax]: the error
+    takes its largest size, alternating, at n + 1 points."""
+    import mpmath as mp
+
+    pts = [zmax * (1 - mp.cos(mp.pi * (2 * i + 1) / (2 * (n + 1)))) / 2 for i in range(n)] + [zmax]
+    grid = [zmax * i / mp.mpf(600) for i in range(1, 601)]
+    h = grid[0]
+    for _ in range(30):
+        a = mp.matrix(n + 1, n + 1)
+        for i, z in enumerate(pts):
+            for j in range(n):
+                a[i, j] = phi(j, z)
+            a[i, n] = (-1) ** i
+        x = mp.lu_solve(a, mp.matrix([f(z) for z in pts]))
+
+        def err(z):
+            return f(z) - sum(x[j] * phi(j, z) for j in range(n))
+
+        peaks = []  # (z, error) of the largest error of each sign run
+        for z in grid:
+            e = err(z)
+            if peaks and (e > 0) == (peaks[-1][1] > 0):
+                if abs(e) > abs(peaks[-1][1]):
+                    peaks[-1] = (z, e)
+            else:
+                peaks.append((z, e))
+        assert len(peaks) == n + 1
+        new = []
+        for z, e in peaks:  # the parabola through three neighbours
+            if z < zmax:
+                lo, hi = err(z - h), err(z + h)
+                z += h * (lo - hi) / (2 * (lo - 2 * e + hi))
+            new.append(z)
+        if max(abs(p - q) for p, q in zip(pts, new)) < mp.mpf(10) ** -25:
+            break
+        pts = new
+    return [x[j] for j in range(n)]
+
+
 def fit_fp64(tmax=0.8, degree=5):
     """cos t ~ 1 + z P(z) and sin t ~ t + t z Q(z), z = t^2, on |t| <= tmax, P and Q of
     degree `degree`: their coefficients rounded to double (highest degree first) and the
@@ -72,32 +113,25 @@ def fit_fp64(tmax=0.8, degree=5):
     import mpmath as mp
 
     mp.mp.dps = 50
-    zmax = mp.mpf(tmax) ** 2
-
-    def pc(z):
-        return (mp.cos(mp.sqrt(z)) - 1) / z if z != 0 else mp.mpf(-0.5)
-
-    def ps(z):
-        return (mp.sin(mp.sqrt(z)) / mp.sqrt(z) - 1) / z if z != 0 else -mp.mpf(1) / 6
-
+    zmax = mp.mpf(str(tmax)) ** 2
     out = {}
-    for name, f, g in (("cos", pc, lambda z, v: 1 + z * v - mp.cos(mp.sqrt(z))),
-                       ("sin", ps, lambda z, v: mp.sqrt(z) * (1 + z * v) - mp.sin(mp.sqrt(z)))):
-        coef = [float(c) for c in mp.chebyfit(f, [0, zmax], degree + 1)]
-        err = 0
-        for i in range(4001):
-            z = zmax * i / 4000
-            err = max(err, abs(g(z, mp.polyval([mp.mpf(c) for c in coef], z))))
-        out[name] = (coef, float(err))
+    for name, f, phi in (("cos", lambda z: mp.cos(mp.sqrt(z)) - 1, lambda j, z: z ** (j + 1)),
+                         ("sin", lambda z: mp.sin(mp.sqrt(z)) - mp.sqrt(z),
+                          lambda j, z: mp.sqrt(z) * z ** (j + 1))):
+        coef = [float(c) for c in remez(f, phi, degree + 1, zmax)]
+        err = max(abs(f(z) - sum(mp.mpf(c) * phi(j, z) for j, c in enumerate(coef)))
+                  for z in (zmax * i / mp.mpf(4000) for i in range(1, 4001)))
+        out[name] = (coef[::-1], float(err))
     return out
 
 
 if __name__ == "__main__":
     import sys
 
-    if len(sys.argv) == 2 and sys.argv[1] == "fp64":
-        for name, (coef, err) in fit_fp64().items():
-            print(f"{name}: max abs error {err:.2e}; coefficients z^5 .. z^0:")
+    if len(sys.argv) in (2, 4) and sys.argv[1] == "fp64":
+        asked = (float(sys.argv[2]), int(sys.argv[3])) if len(sys.argv) == 4 else ()
+        for name, (coef, err) in fit_fp64(*asked).items():
+            print(f"{name}: max abs error {err:.2e}; coefficients, highest degree first:")
             print("  " + ", ".join(f"{c!r}" for c in coef))
         sys.exit(0)
     args = [float(sys.argv[1]), int(sys.argv[2]), int(sys.argv[3])] if len(sys.argv) == 4 else [0.8, 4, 3]
