@@ -25,7 +25,7 @@ namespace bempp_b200 {
 
 void build_singular_pairs(GridT& g, SingularPairList& out);
 void build_tiles(const SpaceT& s, int tile, std::vector<int>& off, std::vector<int>& dofs,
-                 std::vector<uint8_t>& ldof, int& max_dofs, int& max_half_dofs,
+                 std::vector<uint8_t>& ldof, int& max_dofs, int most[2],
                  std::vector<uint8_t>& inc_off, std::vector<uint8_t>& inc_ent);
 int scatter_tile_cells();
 cudaError_t launch_convert_to_single(const double* src, void* dst, size_t n_reals,
@@ -207,11 +207,11 @@ void ensure_space_device(SpaceT& s, int device) {
   std::vector<uint8_t> ldof;
   s.tile_cells = scatter_tile_cells();
   std::vector<uint8_t> inc_off, inc_ent;
-  build_tiles(s, s.tile_cells, off, tdofs, ldof, s.max_tile_dofs, s.max_chunk_dofs, inc_off,
-              inc_ent);
+  build_tiles(s, s.tile_cells, off, tdofs, ldof, s.max_tile_dofs, s.most_dofs, inc_off, inc_ent);
   s.d_tile_inc_off.upload(inc_off);
   s.d_tile_inc_ent.upload(inc_ent);
   s.ntiles = static_cast<int>(off.size()) - 1;
+  s.mean_tile_dofs = s.ntiles > 0 ? off.back() / s.ntiles : 0;
   s.d_tile_off.upload(off);
   s.d_tile_dofs.upload(tdofs);
   s.d_cell_ldof.upload(ldof);
@@ -235,7 +235,8 @@ SpaceTiles space_tiles(const SpaceT& s) {
   t.tile_cells = s.tile_cells;
   t.ntiles = s.ntiles;
   t.max_tile_dofs = s.max_tile_dofs;
-  t.max_chunk_dofs = s.max_chunk_dofs;
+  for (int i = 0; i < 2; ++i) t.most_dofs[i] = s.most_dofs[i];
+  t.mean_tile_dofs = s.mean_tile_dofs;
   t.tile_dof_off = s.d_tile_off.as<int>();
   t.tile_dofs = s.d_tile_dofs.as<int>();
   t.cell_ldof = s.d_cell_ldof.as<uint8_t>();

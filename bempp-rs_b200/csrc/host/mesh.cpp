@@ -334,13 +334,13 @@ void build_singular_pairs(GridT& g, SingularPairList& out) {
 
 // Tile layout for the scatter kernel: tiles of `tile` consecutive cells, their sorted
 // unique DOFs, and each cell's DOFs as indices into its tile's list.
-// max_half_dofs: the most DOFs of half a tile.
+// most: the most DOFs of half a tile and of a quarter.
 // Also the incidence of each tile's local DOFs: for local DOF d of tile t, the entries
 // inc_ent[t * 3 * tile + k], k in [inc_off[t * (3 * tile + 1) + d], ... + d + 1), each
 // b * tile + c for the cell c of the tile whose local basis function b is DOF d (cells
 // ascending, then b).
 void build_tiles(const SpaceT& s, int tile, std::vector<int>& off, std::vector<int>& dofs,
-                 std::vector<uint8_t>& ldof, int& max_dofs, int& max_half_dofs,
+                 std::vector<uint8_t>& ldof, int& max_dofs, int most[2],
                  std::vector<uint8_t>& inc_off, std::vector<uint8_t>& inc_ent) {
   const int64_t nc = s.grid->ncells;
   const int nb = s.nbasis;
@@ -348,7 +348,7 @@ void build_tiles(const SpaceT& s, int tile, std::vector<int>& off, std::vector<i
   off.assign(ntiles + 1, 0);
   dofs.clear();
   ldof.assign(nc * nb, 0);
-  max_dofs = max_half_dofs = 0;
+  max_dofs = most[0] = most[1] = 0;
   // the DOF incidence serves the P1 / DP1 gather of the tiled kernels only (degree-2
   // spaces use the generic pair kernel)
   const bool incidence = nb <= 3;
@@ -372,9 +372,14 @@ void build_tiles(const SpaceT& s, int tile, std::vector<int>& off, std::vector<i
     off[t + 1] = static_cast<int>(dofs.size());
     max_dofs = std::max<int>(max_dofs, static_cast<int>(local.size()));
     for (int64_t h = c0; h < c1; h += tile / 2) {
-      std::bitset<256> used;  // at most 6 * 32 DOFs per tile
-      for (int64_t i = h * nb; i < std::min(h + tile / 2, c1) * nb; ++i) used.set(ldof[i]);
-      max_half_dofs = std::max<int>(max_half_dofs, static_cast<int>(used.count()));
+      std::bitset<256> half;  // at most 6 * 32 DOFs per tile
+      for (int64_t q = h; q < std::min(h + tile / 2, c1); q += tile / 4) {
+        std::bitset<256> quarter;
+        for (int64_t i = q * nb; i < std::min(q + tile / 4, c1) * nb; ++i) quarter.set(ldof[i]);
+        most[1] = std::max<int>(most[1], static_cast<int>(quarter.count()));
+        half |= quarter;
+      }
+      most[0] = std::max<int>(most[0], static_cast<int>(half.count()));
     }
     if (!incidence) continue;
     // incidence (counting sort of the tile's (cell, basis) entries by local DOF)

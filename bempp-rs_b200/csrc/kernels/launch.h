@@ -82,7 +82,8 @@ struct SpaceTiles {
   int tile_cells;           // cells per tile
   int ntiles;
   int max_tile_dofs;
-  int max_chunk_dofs;       // most DOFs of 16 consecutive cells (half a tile)
+  int most_dofs[2];         // most DOFs of half a tile, of a quarter (16 and 8 cells)
+  int mean_tile_dofs;
   const int* tile_dof_off;  // ntiles + 1
   const int* tile_dofs;     // global DOF numbers of each tile, ascending
   const uint8_t* cell_ldof; // ncells * nbasis local (in-tile) DOF indices

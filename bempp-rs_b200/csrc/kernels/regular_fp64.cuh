@@ -1541,20 +1541,23 @@ inline bool has_orbit_form(const RegularRule& r) {
 }
 
 constexpr int kSMs = 148;
+constexpr int kAccumulatorBytes = 20 << 10;  // per warp, at most (see set_accumulator)
 
 template <int KER, int NBS, bool DIRECT, bool PAIRED>
 inline void set_accumulator(Shape& sh, const SpaceTiles& tt, const SpaceTiles& st) {
-  // accumulators of up to 12 KB per warp: three CTAs per SM stay resident; larger ones
-  // (discontinuous P1, meshes whose tiles touch many DOFs) are replaced by direct adds
+  // accumulators of up to 20 KB per warp (the other arrays take 7 to 11 KB of a warp: two CTAs of
+  // four warps stay resident with 17 KB, one with more); larger ones (discontinuous P1, meshes whose
+  // tiles touch many DOFs) are replaced by direct adds, which cost less than the flushes of
+  // shorter chunks (20,480 triangles in a mesher's order, 45 DOFs per tile on average and 77 at most,
+  // Laplace double layer P1: 16.3 ms with direct adds, 23.2 with accumulators for eight cells)
   sh.cap = 0;
   sh.gather = 0;
   if (!DIRECT) {
-    const int chunk_dofs = std::min(st.max_tile_dofs, sh.ns * NBS);
-    // (a shorter chunk lies within one of kChunk cells)
-    sh.cap = tt.max_tile_dofs * std::min(chunk_dofs, st.max_chunk_dofs);
+    // (a shorter chunk lies within one of eight or sixteen cells)
+    sh.cap = tt.max_tile_dofs * std::min(sh.ns * NBS, st.most_dofs[sh.ns > 8 ? 0 : 1]);
     const size_t bytes = sizeof(double) * static_cast<size_t>(sh.cap) * (KER == kHelmholtz ? 2 : 1) *
                          (PAIRED ? 2 : 1);
-    sh.gather = bytes <= (size_t(20) << 10) ? 1 : 0;
+    sh.gather = bytes <= kAccumulatorBytes ? 1 : 0;
     if (!sh.gather) sh.cap = 0;
   }
 }
@@ -1599,8 +1602,10 @@ cudaError_t launch_shape(const CellSet& test, const SpaceTiles& tt, const CellSe
 // Trial cells per CTA of the 6-point rule's kernels (`tiles`: CTAs that whole tiles would take).
 // A CTA costs its staging, incidence and flush (about `fixed` trial cells' time per wave of
 // the CTAs that an SM holds, and the adds of its block); a trial cell costs one unit per CTA
-// on the SM, but not less than four (one warp's latency).  The least estimate, longer chunks on
-// ties.  B200, shorter chunks until 888 CTAs -> this: 640 triangles, one space, Laplace double
+// on the SM, but not less than four (one warp's latency), a fifth more where it adds directly, and
+// two thirds more where one CTA fills the SM's shared memory (a torus of 20,480 triangles in rows,
+// 34 DOFs per tile, Helmholtz double layer P1, k = 8: chunks of sixteen 63.9 ms, of eight 42.7).
+// The least estimate, longer chunks on ties.  B200, shorter chunks until 888 CTAs -> this: 640 triangles, one space, Laplace double
 // layer P1 53 -> 35 us, single layer DP0 27 -> 19; 1,280: double layer 91 -> 77; two bodies of
 // 800 and 700, hypersingular 46 -> 41; Helmholtz, k = 10: 1,280 hypersingular 168 -> 142, two
 // bodies double layer 156 -> 123.
@@ -1619,7 +1624,9 @@ inline int orbit_chunk(long long tiles, Shape sh, const SpaceTiles& tt, const Sp
     const long long resident = std::max<long long>(
         1, std::min<long long>(min_ctas<true, KER, OP, NBT, NBS, PAIRED>(), (size_t(227) << 10) / smem));
     const long long n = (tiles * (kTile / ns) + kSMs - 1) / kSMs;  // CTAs of the fullest SM
-    const long long cost = (n + resident - 1) / resident * fixed + n * adds + ns * std::max(4LL, n);
+    const bool direct_adds = !DIRECT && !sh.gather;
+    const long long cells = ns * std::max(4LL, n) * (direct_adds ? 6 : 5) / 5 * (resident == 1 && n > 1 ? 5 : 3) / 3;
+    const long long cost = (n + resident - 1) / resident * fixed + (direct_adds ? 0 : n * adds) + cells;
     if (ns == kChunk || cost < least) {
       least = cost;
       best = ns;
