@@ -1195,6 +1195,9 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
     if (!((skip >> js) & 1u) && close_pair(p, T.G(rR, it) + S.G(rR, js), rule.reach)) close |= 1u << js;
   }
   skip |= close;
+  // not in a register through the loop (20,480 triangles, double layer P1: 13.76 -> 13.61 ms): in the
+  // lane's own rR, which nothing reads from here on (SPLIT: the warps share the tile)
+  if constexpr (!SPLIT) reinterpret_cast<unsigned*>(T.geo + rR * kTile)[2 * it] = close;
   int rows[NBT];  // direct adds: the lane's test DOFs
   if constexpr (!DIRECT) {
     if (!sh.gather)
@@ -1417,6 +1420,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<ORBITS, KER, OP, NBT, NBS, 
       }
     }
   }
+  if constexpr (!SPLIT) close = reinterpret_cast<volatile unsigned*>(T.geo + rR * kTile)[2 * it];
   if (__any_sync(0xffffffffu, close != 0u))
     add_close_pairs<KER, OP, NBT, NBS, DIRECT, PAIRED, SPLIT>(
         T, it, S, close, rt, Q, warp, k, DIRECT ? nullptr : tt.cell_dofs + static_cast<int64_t>(ti0) * NBT,
