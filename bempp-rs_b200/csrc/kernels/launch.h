@@ -64,7 +64,7 @@ struct RegularArgs {
   NearArgs near{};       // mixed: near field (null: near pairs found per pair in the kernel)
   int symmetric = 0;     // 1: test and trial are one space and the operator is symmetric
                          // (SL, HS): only tile pairs (tx >= sy) are computed, then mirrored;
-                         // 2: one P1 / DP1 space, DL or ADL, 6-point rule (Helmholtz:
+                         // 2: one P1 / DP1 space, DL or ADL (mixed: 6-point rule and, Helmholtz,
                          // phases within the polynomial range): tile pairs (tx >= sy),
                          // each integrated in both orders
   int trial_tile0 = 0;   // first trial tile of this launch

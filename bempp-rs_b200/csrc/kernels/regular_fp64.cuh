@@ -39,9 +39,9 @@
 //
 // Regular part on a B200, coordinate differences in 32 x 32 tiles per CTA -> this form:
 //   20,480 triangles, 6-point rule: Laplace single layer DP0 6.55 -> 5.05 ms, double layer P1
-//   (both orders of a pair at once) 17.7 -> 13.2, hypersingular P1 9.5 -> 7.3; Helmholtz
-//   k = 8 single layer DP0 15.8 -> 12.6, double layer P1 39.8 -> 35.7, hypersingular P1
-//   28.0 -> 21.1; 5,120 triangles, k = 8 (phases beyond 0.8): single layer 1.61 -> 1.18;
+//   (both orders of a pair at once) 17.7 -> 13.3, hypersingular P1 9.5 -> 7.3; Helmholtz
+//   k = 8 single layer DP0 15.8 -> 12.5, double layer P1 39.8 -> 35.9, hypersingular P1
+//   28.0 -> 21.4; 5,120 triangles, k = 8 (phases beyond 0.8): single layer 1.61 -> 1.18;
 //   2,048 triangles, 37-point rule: double layer P1 10.7 -> 4.0 (both orders at once);
 //   80 triangles, 37-point rule: single layer DP0 0.374 -> 0.021.
 // In FP64 issue slots the double layer needs about 19 per point pair for both orders (26

@@ -26,7 +26,7 @@
 //
 // Three ellipsoids of 5,120, 1,280 and 320 triangles, 8 wavenumbers up to 20, B200, each
 // wavenumber by itself -> this form: far pairs 6.6 -> 1.7 ms, vertex-sharing pairs 2.3 -> 0.8, the
-// whole call 8.2 -> 2.8; error against FP64 4.2e-8 -> 3.9e-8 (the phase k r0 and its rotation are
+// whole call 8.1 to 8.5 -> 2.7 to 3.1; error against FP64 4.2e-8 -> 3.9e-8 (the phase k r0 and its rotation are
 // FP64 here).  The far pairs issue in 60% of the cycles (16 warps per SM at 128 registers).
 #include <algorithm>
 #include <cmath>
