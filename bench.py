@@ -55,15 +55,26 @@ Q_REGULAR = 6
 ORDER = 4
 SEED = 20480
 
-# Algorithmic FLOPs per regular cell pair at Q = 6 (36 point pairs): kernel evaluation
-# plus basis accumulation, transcendental functions counted as 1, per-cell constants
-# hoisted (P1 x P1 uses the factorised sum U_b(p) = sum_q K psi_b w_q).
+# FLOPs per integrated regular cell pair at Q = 6 (36 point pairs; add, mul = 1, FMA = 2, square
+# roots, sines and cosines = 1), as the kernels of each precision do them.  FP64: distances as a
+# bilinear form from the centroids (2 operations per point pair), P1 sums per rule orbit, the
+# double layer's two orders from one kernel value (half of the pair's work each).  Mixed: FP32
+# differences of coordinates, each order by itself.
 FLOPS_PER_PAIR = {
-    ("laplace", "single_layer", "dp0"): 396,
-    ("laplace", "double_layer", "p1"): 990,
-    ("laplace", "adjoint_double_layer", "p1"): 990,
-    ("laplace", "hypersingular", "p1"): 459,
-    ("helmholtz", "single_layer", "dp0"): 720,
+    "fp64": {
+        ("laplace", "single_layer", "dp0"): 302,
+        ("laplace", "double_layer", "p1"): 444,
+        ("laplace", "adjoint_double_layer", "p1"): 444,
+        ("laplace", "hypersingular", "p1"): 298,
+        ("helmholtz", "single_layer", "dp0"): 627,
+    },
+    "mixed": {
+        ("laplace", "single_layer", "dp0"): 396,
+        ("laplace", "double_layer", "p1"): 990,
+        ("laplace", "adjoint_double_layer", "p1"): 990,
+        ("laplace", "hypersingular", "p1"): 459,
+        ("helmholtz", "single_layer", "dp0"): 720,
+    },
 }
 
 # DRAM bytes (read + write) per launch of the dominant regular kernel, from one ncu capture
@@ -333,7 +344,7 @@ def helmholtz_sl_fp64_vs_mixed(args):
         # algorithmic FLOPs of the integrated regular pairs over the phase time (mixed: the
         # FP32 far pairs, with the FP64 near and singular kernels of that phase in the time)
         nreg = len(wl.cells) ** 2 - singular_pair_count(wl.cells)
-        fl = FLOPS_PER_PAIR[("helmholtz", "single_layer", "dp0")] * integrated_pairs("single_layer", nreg)
+        fl = FLOPS_PER_PAIR[prec][("helmholtz", "single_layer", "dp0")] * integrated_pairs("single_layer", nreg)
         peak = fma_peak(fp64=prec == "fp64")
         ach = fl / (res[prec]["regular_ms"] * 1e-3) / 1e12 if res[prec]["regular_ms"] else None
         res[prec]["roofline"] = {"bound": "fp64" if prec == "fp64" else "fp32", "achieved": ach,
@@ -666,7 +677,7 @@ def run_ours(args):
     for name, ph in phases.items():
         key = (w["kernel"], name, w["space"])
         reg_ms = ph[2] if len(ph) > 2 else float("nan")
-        fl = FLOPS_PER_PAIR.get(key)
+        fl = FLOPS_PER_PAIR[args.precision].get(key)
         per_op[name] = {"regular_ms": reg_ms, "phase_ms": ph,
                         "pairs_integrated": integrated_pairs(name, nreg),
                         "tflops": fl * integrated_pairs(name, nreg) / (reg_ms * 1e-3) / 1e12
